@@ -15,7 +15,7 @@
 //                       same pass already changed)
 //   amr_apply_kernel    the decisions applied (depth and bed of the parent), zs
 //                       recomputed on the prolongated halo
-//   amr_flux2_kernel    tile with its outer stencil ring, gradients, wet-slope
+//   amr_flux_kernel    tile with its outer stencil ring, gradients, wet-slope
 //                       reset, faces with the coarse/fine source substitution,
 //                       cell dtmax and the block minimum (predictor only);
 //                       faces written to the stage face arrays
@@ -40,7 +40,7 @@ namespace BGF_VARIANT {
 
 #include "bgf_stage.cuh"
 #include "bgf_pair.cuh"
-#include "bgf_flow2.cuh"
+#include "bgf_quad.cuh"
 
 __device__ __forceinline__ bool has_coarser_side(const int* nbr, int nbm, const int* lv, int ib)
 {
@@ -306,52 +306,53 @@ template <class T> struct AmrOcc {
     static constexpr int flux = sizeof(T) == 4 ? 6 : 3;
 };
 
-// The multi-level flux kernel, in the two-cells-per-thread layout of the single-level kernels
-// (bgf_flow2.cuh): 128 threads per block, thread (x, p) owning cells (x, 2p) and
-// (x, 2p+1).  The tile comes from the stage tile W (interior and ring 1, whose
-// halos the chain filled) and the outer ring rules (ring 2); gradients, wet-slope
-// reset and faces are the single-level kernels' own, with the coarse/fine source
-// substitution on the sides whose neighbour is coarser.  The faces go to the stage
-// face arrays in the layout amr_update_kernel reads.  The same operations in the
-// same order as the reference's FlowCPU: the exact build matches the oracle bit for bit.
+// Cells of a pair that a thread of the flux kernel owns (as quad_lanes in bgf_flow.cu).
+template <class T> __host__ __device__ constexpr int amr_lanes() { return sizeof(T) == 8 ? 1 : 2; }
+
+// The multi-level flux kernel, in the layout of the single-level kernels (bgf_quad.cuh).
+// The tile comes from the stage tile W (interior and ring 1, whose halos the chain
+// filled) and the outer ring rules (ring 2); gradients, wet-slope reset and faces are the
+// single-level kernels' own, with the coarse/fine source substitution on the sides whose
+// neighbour is coarser.  The faces go to the stage face arrays in the layout
+// amr_update_kernel reads.  The same operations in the same order as the reference's
+// FlowCPU: the exact build matches the oracle bit for bit.
 template <class T, int ENGINE>
-__global__ void __launch_bounds__(NT2, AmrOcc<T>::flux) amr_flux2_kernel(DevModel<T> m, AmrDev<T> a, StepParams<T> p0,
-                                                                            int parity, int stage)
+__global__ void __launch_bounds__(Quad<T, amr_lanes<T>()>::NT, AmrOcc<T>::flux)
+    amr_flux_kernel(DevModel<T> m, AmrDev<T> a, StepParams<T> p0, int parity, int stage)
 {
-    using V = V2<T>;
-    extern __shared__ __align__(16) unsigned char smem_raw2[];
-    Smem2<T>& s = *reinterpret_cast<Smem2<T>*>(smem_raw2);
+    constexpr int LANES = amr_lanes<T>(), NT = Quad<T, LANES>::NT;
+    using V = typename ValOf<T, LANES>::V;
+    extern __shared__ __align__(16) unsigned char smem_rawq[];
+    SmemQ<T, LANES>& s = *reinterpret_cast<SmemQ<T, LANES>*>(smem_rawq);
     __shared__ SubFaces<T> sub;
     const int tid = threadIdx.x;
-    const int w4 = tid >> 5, lane = tid & 31;
-    const int x = lane & 15;
-    const int py = (w4 & 1) + 4 * (w4 >> 1) + 2 * (lane >> 4);
-    const int y = 2 * py;
+    const Place<T, LANES> at(tid, blockIdx.x);
     const int ib = m.active[blockIdx.x];
     const int sc = scen_of(m, ib);
     const StepParams<T>& p = m.sparams ? m.sparams[sc] : p0;
     const int nbm = m.nblkmem;
     T* const* W = a.W[stage];
     const size_t base = (size_t)ib * 324;
-    const T* zbt = m.zb + base;
     // every load that does not depend on the block's time slot is issued before it
-    // arrives: the bed tile and gradients, the own pair and ring 1 from the stage
-    // tile, the coarse/fine sources, and ring 2 inside a coarser neighbour's patch
-    load_bed2<T>(s, zbt, tid);
-    const BedGrad<T> bg = load_bedgrad<T, ENGINE>(m, ib, tid, x, y);
+    // arrives: the bed and its gradients, the own cells and ring 1 from the stage tile, the
+    // coarse/fine sources, and ring 2 inside a coarser neighbour's patch
+    const V zb = own_of<V>(m.zb + base, hi18(at.x, at.r), 8 * 18, at.l);
+    BedGradQ<T, LANES> bg;
+    load_bedgrad_q<T, ENGINE, LANES>(m, ib, at, bg);
     V c[4];
 #pragma unroll
-    for (int v = 0; v < 4; v++) c[v] = V{W[v][base + hi18(x, y)], W[v][base + hi18(x, y + 1)]};
+    for (int v = 0; v < 4; v++) c[v] = own_of<V>(W[v] + base, hi18(at.x, at.r), 8 * 18, at.l);
     CellRule<T> r{};  // ring 2 (threads 64..127)
-    int o2 = 0;
+    int rx = 0, ry = 0;
     if (tid < 64) {
         // ring 1 (the block's halo, corners excluded) and the coarse/fine substitution
         const int sd = tid >> 4, t = tid & 15;
         int hx, hy;
         halo_xy(sd, t, hx, hy);
-        const int c18 = hi18(hx, hy), o = p2t(hx, hy);
+        const size_t c18 = base + hi18(hx, hy);
 #pragma unroll
-        for (int v = 0; v < 4; v++) s.t[v][o] = W[v][base + c18];
+        for (int v = 0; v < 4; v++) BGF_ROW(s.t[v], pt, hx, hy) = W[v][c18];
+        BGF_ROW(s.zb, pz, hx, hy) = m.zb[c18];
         int pb, px, pyy;
         const bool coarse = parent_cell(m.nbr, nbm, m.level, ib, sd, t, pb, px, pyy);
         if (t == 0) sub.on[sd] = coarse ? 1 : 0;
@@ -359,33 +360,28 @@ __global__ void __launch_bounds__(NT2, AmrOcc<T>::flux) amr_flux2_kernel(DevMode
             sub.h[sd][t] = W[0][(size_t)pb * 324 + hi18(px, pyy)];
             sub.z[sd][t] = a.zb[(size_t)pb * 324 + hi18(px, pyy)];
         }
-    } else {
+    } else if (tid < 128) {
         // ring 2: the outer stencil values of the halo gradients
         const int k = tid - 64;
         const int sd = k >> 4, t = k & 15;
         r = outer_rule<T>(m.nbr, nbm, m.level, ib, sd, t);
-        int rx, ry;
         halo_xy(sd, t, rx, ry);
         if (sd == 0) rx = -2;
         else if (sd == 1) rx = BW + 1;
         else if (sd == 2) ry = -2;
         else ry = BW + 1;
-        o2 = p2t(rx, ry);
         if (r.kind == 3) {
             // inside a coarser neighbour's 2x2 patch, which may reach into its halo:
             // that neighbour has a finer neighbour, so it runs this chain and its
             // stage tile is filled
 #pragma unroll
-            for (int v = 0; v < 4; v++) s.t[v][o2] = rule_eval(r, Acc324<T>{W[v]});
+            for (int v = 0; v < 4; v++) BGF_ROW(s.t[v], pt, rx, ry) = rule_eval(r, Acc324<T>{W[v]});
         }
     }
     const TimeState ts = m.time[2 * sc + parity];
-    if (!step_live(ts)) {
-        bed_wait();  // (no bed copy outlives the block)
-        return;
-    }
+    if (!step_live(ts)) return;
     const T delta = calcres<T>(p.delta0, m.level[ib]);
-    if (tid >= 64 && r.kind != 3) {
+    if (tid >= 64 && tid < 128 && r.kind != 3) {
         // ring 2 at interior cells of this block or of a same-level or finer
         // neighbour, read as the stage reads any cell (the neighbour may run the
         // single-level kernels and have no stage tile): the state of the step
@@ -399,45 +395,29 @@ __global__ void __launch_bounds__(NT2, AmrOcc<T>::flux) amr_flux2_kernel(DevMode
         }
 #pragma unroll
         for (int v = 0; v < 4; v++)
-            s.t[v][o2] = r.kind == 0 ? cv[0][v] : (T)0.25 * (cv[0][v] + cv[1][v] + cv[2][v] + cv[3][v]);
+            BGF_ROW(s.t[v], pt, rx, ry) = r.kind == 0 ? cv[0][v] : (T)0.25 * (cv[0][v] + cv[1][v] + cv[2][v] + cv[3][v]);
     }
-    const int ct = p2t(x, y);
-#pragma unroll
-    for (int k = 0; k < 4; k++) st2<T>(s.t[k], ct, c[k]);
-    bed_wait();
+    store_own<T, LANES>(s, at, c, zb);
     __syncthreads();
-    V xm[4], gxo[4], gyo[4];
-    T ym[4];
-    gradients2<T, ENGINE>(s, bg, p.theta, delta, tid, x, py, c, xm, ym, gxo, gyo);
-    __syncthreads();
-    V cdt = faces2<T, ENGINE, false, true>(s, p, delta, tid, x, py, c, xm, ym, gxo, gyo, (T)0, &sub);
-    if (stage == 0) {
-        cdt = finite_dt2<T>(c[VH], c[VU], c[VV], cdt);
-        T v = cdt.b < cdt.a ? cdt.b : cdt.a;
-        for (int o = 16; o > 0; o >>= 1) {
-            const T q = __shfl_xor_sync(0xffffffffu, v, o);
-            v = q < v ? q : v;
-        }
-        if (lane == 0) s.red[w4] = v;
-    }
-    __syncthreads();  // every face written (the right column and top row by warp 0)
+    OwnFlux<V> own;
+    T amax = tile_faces<T, ENGINE, LANES, false, true, true>(s, p, delta, at, c, zb, bg, true, own, (T)0, &sub);
+    if (stage == 0) warp_max<T, LANES>(s, tid, finite_speed(c[VH], c[VU], c[VV], amax));
+    __syncthreads();  // every face written
     // faces to the stage face arrays: X faces at fxi(x, y) (x = 16 after the 256
     // interior faces), Y faces at fyi(x, y)
     const size_t fb = (size_t)ib * NFX;
-    for (int k = tid; k < NFX; k += NT2) {
-        const int ox = k < 256 ? p2fx(k & 15, k >> 4) : p2fx(BW, k - 256);
-        const int oy = p2fy(k & 15, k >> 4);
-#pragma unroll
-        for (int v = 0; v < 4; v++) {
-            a.F[v][fb + k] = s.fx[v][ox];
-            a.F[4 + v][fb + k] = s.fy[v][oy];
-        }
+    for (int k = tid; k < NFX; k += NT) {
+        const int fx = k < 256 ? k & 15 : BW, fy = k < 256 ? k >> 4 : k - 256, gy = k >> 4;
+        a.F[0][fb + k] = BGF_ROW(s.fx[0], pfx, fx, fy);
+        a.F[1][fb + k] = BGF_ROW(s.fxq(), pfx, fx, fy);
+        a.F[2][fb + k] = BGF_ROW(s.fx[1], pfx, fx, fy);
+        a.F[3][fb + k] = BGF_ROW(s.fx[2], pfx, fx, fy);
+        a.F[4][fb + k] = BGF_ROW(s.fy[0], pfy, k & 15, gy);
+        a.F[5][fb + k] = BGF_ROW(s.fyq(), pfy, k & 15, gy);
+        a.F[6][fb + k] = BGF_ROW(s.fy[1], pfy, k & 15, gy);
+        a.F[7][fb + k] = BGF_ROW(s.fy[2], pfy, k & 15, gy);
     }
-    if (stage == 0 && tid == 0) {
-        T b = s.red[0];
-        for (int k = 1; k < NT2 / 32; k++) b = s.red[k] < b ? s.red[k] : b;
-        atomicMin(&m.dtmin[2 * sc + parity], dt_bits(b));
-    }
+    if (stage == 0 && tid == 0) block_dt<T, LANES>(s, p, delta, &m.dtmin[2 * sc + parity]);
 }
 
 template <class T, int ENGINE>
@@ -640,8 +620,8 @@ template <class T> static size_t amr_smem() { return sizeof(Smem<T>); }
 
 template <class T, int ENGINE> static cudaError_t amr_configure_engine()
 {
-    cudaError_t e = cudaFuncSetAttribute(amr_flux2_kernel<T, ENGINE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem2_pred<T>());
+    cudaError_t e = cudaFuncSetAttribute(amr_flux_kernel<T, ENGINE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)sizeof(SmemQ<T, amr_lanes<T>()>));
     if (e != cudaSuccess) return e;
     return cudaFuncSetAttribute(amr_update_kernel<T, ENGINE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                 (int)amr_smem<T>());
@@ -670,11 +650,13 @@ int launch_amr_stage(const DevModel<T>& m, const AmrDev<T>& a, const StepParams<
         }
     }
     amr_apply_kernel<T><<<n, 64, 0, st>>>(m, a, p, parity, stage);
+    constexpr int nt = Quad<T, amr_lanes<T>()>::NT;
+    constexpr size_t smq = sizeof(SmemQ<T, amr_lanes<T>()>);
     if (engine == 1) {
-        amr_flux2_kernel<T, 1><<<n, NT2, smem2_pred<T>(), st>>>(m, a, p, parity, stage);
+        amr_flux_kernel<T, 1><<<n, nt, smq, st>>>(m, a, p, parity, stage);
         amr_update_kernel<T, 1><<<n, NTHREADS, amr_smem<T>(), st>>>(m, a, p, parity, stage);
     } else {
-        amr_flux2_kernel<T, 2><<<n, NT2, smem2_pred<T>(), st>>>(m, a, p, parity, stage);
+        amr_flux_kernel<T, 2><<<n, nt, smq, st>>>(m, a, p, parity, stage);
         amr_update_kernel<T, 2><<<n, NTHREADS, amr_smem<T>(), st>>>(m, a, p, parity, stage);
     }
     return launches + 3;

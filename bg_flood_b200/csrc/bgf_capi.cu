@@ -114,9 +114,9 @@ struct bgf_handle {
     bool has_blocks = false, has_bed = false, has_state = false, has_cf = false, has_rainmask = false;
     int nseg_dev = 0, rain_n_dev = 0;
     int64_t launches = 0;
-    // graph of two consecutive steps (parities p, p^1)
+    // graphs of two and of kLongRun consecutive steps from parity p (built when first used)
     cudaGraphExec_t graph[2] = {nullptr, nullptr};
-    bool graph_valid = false;
+    cudaGraphExec_t graph_long[2] = {nullptr, nullptr};
     // graph of one bgf_flow_step per parity: time-slot upload, the step, result download
     cudaGraphExec_t step_graph[2] = {nullptr, nullptr};
     int step_graph_launches[2] = {0, 0};
@@ -235,6 +235,7 @@ template <class T> static DevModel<T> dev_model(bgf_handle* h)
     m.checklev = 0;
     m.datum = h->split ? (const T*)h->d_datum : nullptr;
     m.gen = h->gen;
+    m.pdl = 1;
     m.regular_nbx = h->amr ? 0 : h->regular_nbx;
     m.regular_nby = h->regular_nby;
     m.regular_magic = h->regular_magic;
@@ -342,12 +343,15 @@ static void free_graphs(bgf_handle* h)
             cudaGraphExecDestroy(h->graph[k]);
             h->graph[k] = nullptr;
         }
+        if (h->graph_long[k]) {
+            cudaGraphExecDestroy(h->graph_long[k]);
+            h->graph_long[k] = nullptr;
+        }
         if (h->step_graph[k]) {
             cudaGraphExecDestroy(h->step_graph[k]);
             h->step_graph[k] = nullptr;
         }
     }
-    h->graph_valid = false;
 }
 
 // Reads a BUQ field of the caller's precision into a T vector.
@@ -1830,32 +1834,53 @@ int bgf_flow_step(bgf_handle* h, bgf_loop* loop)
     return finish_step(h, loop, *(const int*)&h->h_misc[1], h->h_time[1]);
 }
 
-static int build_graphs(bgf_handle* h)
+// Steps of a long run graph.  Inside a graph the step kernels overlap at their ends
+// (programmatic dependent launch); between two graphs they do not.  A run replays long
+// graphs for as many steps as fit and graphs of two for the rest.
+constexpr int kLongRun = 16;
+
+static int build_run_graph(bgf_handle* h, int p0, int steps, cudaGraphExec_t* out)
 {
-    for (int k = 0; k < 2; k++)  // the run graphs only; the single-step graphs stay valid
-        if (h->graph[k]) {
-            cudaGraphExecDestroy(h->graph[k]);
-            h->graph[k] = nullptr;
-        }
-    for (int p0 = 0; p0 < 2; p0++) {
-        cudaGraph_t g;
-        BGF_CUDA(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
-        int n = 0;
-        for (int k = 0; k < 2; k++) n += h->dbl ? enqueue_step<double>(h, p0 ^ k) : enqueue_step<float>(h, p0 ^ k);
-        h->steps_launches = n / 2;
-        cudaError_t e = cudaStreamEndCapture(h->stream, &g);
-        if (e != cudaSuccess) {
-            g_last_error = std::string("graph capture: ") + cudaGetErrorString(e);
-            return BGF_ECUDA;
-        }
-        e = cudaGraphInstantiate(&h->graph[p0], g, 0);
-        cudaGraphDestroy(g);
-        if (e != cudaSuccess) {
-            g_last_error = std::string("graph instantiate: ") + cudaGetErrorString(e);
-            return BGF_ECUDA;
-        }
+    cudaGraph_t g;
+    BGF_CUDA(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
+    int n = 0;
+    for (int k = 0; k < steps; k++)
+        n += h->dbl ? enqueue_step<double>(h, p0 ^ (k & 1)) : enqueue_step<float>(h, p0 ^ (k & 1));
+    h->steps_launches = n / steps;
+    cudaError_t e = cudaStreamEndCapture(h->stream, &g);
+    if (e != cudaSuccess) {
+        g_last_error = std::string("graph capture: ") + cudaGetErrorString(e);
+        return BGF_ECUDA;
     }
-    h->graph_valid = true;
+    e = cudaGraphInstantiate(out, g, 0);
+    cudaGraphDestroy(g);
+    if (e != cudaSuccess) {
+        *out = nullptr;
+        g_last_error = std::string("graph instantiate: ") + cudaGetErrorString(e);
+        return BGF_ECUDA;
+    }
+    return BGF_OK;
+}
+
+// The graphs that `steps` steps (rounded up to whole graphs of two) from parity p0 take:
+// *nlong and *npair of them, built when first needed.
+static int prepare_run(bgf_handle* h, int p0, int steps, int* nlong, int* npair)
+{
+    const int pairs = std::max(1, (steps + 1) / 2);
+    // (a multi-level step is up to 18 launches, most of them not chained: a long graph would
+    // cost more to build after each refinement pass than it saves)
+    *nlong = h->amr ? 0 : pairs / (kLongRun / 2);
+    *npair = h->amr ? pairs : pairs % (kLongRun / 2);
+    int rc = BGF_OK;
+    if (*nlong && !h->graph_long[p0] && (rc = build_run_graph(h, p0, kLongRun, &h->graph_long[p0]))) return rc;
+    if (*npair && !h->graph[p0]) rc = build_run_graph(h, p0, 2, &h->graph[p0]);
+    return rc;
+}
+
+static int launch_run(bgf_handle* h, int p0, int nlong, int npair)
+{
+    for (int b = 0; b < nlong; b++) BGF_CUDA(cudaGraphLaunch(h->graph_long[p0], h->stream));
+    for (int b = 0; b < npair; b++) BGF_CUDA(cudaGraphLaunch(h->graph[p0], h->stream));
     return BGF_OK;
 }
 
@@ -1865,10 +1890,6 @@ int bgf_run(bgf_handle* h, bgf_loop* loop, double endtime, double outputtimestep
     if (rc) return rc;
     if (!loop || maxsteps < 0) return BGF_EINVAL;
     if (nsteps) *nsteps = 0;
-    if (!h->graph_valid) {
-        rc = build_graphs(h);
-        if (rc) return rc;
-    }
     rc = write_time_slot(h, loop, endtime, outputtimestep, maxsteps);
     if (rc) return rc;
     const int p0 = h->parity;
@@ -1880,11 +1901,12 @@ int bgf_run(bgf_handle* h, bgf_loop* loop, double endtime, double outputtimestep
         double remaining = (endtime - ts.totaltime) / (dtguess > 0 ? dtguess : 1.0);
         long long left = (long long)maxsteps - ts.nstep;
         long long want = (long long)std::min<double>(remaining * 1.02 + 2.0, (double)left);
-        int batch = (int)std::max<long long>(1, std::min<long long>((want + 1) / 2, 512));
+        int nlong = 0, npair = 0;
+        if ((rc = prepare_run(h, p0, (int)std::max<long long>(1, std::min<long long>(want, 1024)), &nlong, &npair))) return rc;
         BGF_CUDA(cudaEventRecord(h->ev0, h->stream));
-        for (int b = 0; b < batch; b++) BGF_CUDA(cudaGraphLaunch(h->graph[p0], h->stream));
+        if ((rc = launch_run(h, p0, nlong, npair))) return rc;
         BGF_CUDA(cudaEventRecord(h->ev1, h->stream));
-        launched += 2LL * h->steps_launches * batch;
+        launched += (int64_t)h->steps_launches * (nlong * kLongRun + 2 * npair);
         // after whole graphs the latest time state is in slot p0
         BGF_CUDA(cudaMemcpyAsync(&h->h_time[1], h->d_time + p0, sizeof(TimeState), cudaMemcpyDeviceToHost, h->stream));
         BGF_CUDA(cudaStreamSynchronize(h->stream));
@@ -2705,12 +2727,13 @@ static int tune_restore(bgf_handle* h, TuneSave& t)
 // current launch shape, from the time slot written by the caller.
 static int tune_time_handle(bgf_handle* h, int steps, double* ms)
 {
-    int rc = build_graphs(h);
-    if (rc) return rc;
     const int p0 = h->parity;
-    BGF_CUDA(cudaGraphLaunch(h->graph[p0], h->stream));
+    int nlong = 0, npair = 0, rc;
+    free_graphs(h);  // (of another launch shape)
+    if ((rc = prepare_run(h, p0, 2, &nlong, &npair)) || (rc = launch_run(h, p0, nlong, npair))) return rc;
+    if ((rc = prepare_run(h, p0, steps, &nlong, &npair))) return rc;
     BGF_CUDA(cudaEventRecord(h->ev0, h->stream));
-    for (int k = 0; k < (steps + 1) / 2; k++) BGF_CUDA(cudaGraphLaunch(h->graph[p0], h->stream));
+    if ((rc = launch_run(h, p0, nlong, npair))) return rc;
     BGF_CUDA(cudaEventRecord(h->ev1, h->stream));
     BGF_CUDA(cudaStreamSynchronize(h->stream));
     float t = 0.f;

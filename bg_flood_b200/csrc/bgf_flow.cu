@@ -20,8 +20,7 @@ namespace BGF_VARIANT {
 
 #include "bgf_stage.cuh"
 #include "bgf_pair.cuh"
-#include "bgf_flow2.cuh"
-#include "bgf_flow3.cuh"
+#include "bgf_quad.cuh"
 
 // ---------------------------------------------------------------- tile assembly
 
@@ -361,7 +360,30 @@ template <class T> __global__ void volume_kernel(DevModel<T> m, T delta0, int cu
 
 // ---------------------------------------------------------------- launchers
 
+constexpr int kOneCellBlocks = 700;
+
 template <class T> size_t smem_bytes() { return sizeof(Smem<T>); }
+
+// Cells of a pair that a thread of the step kernels owns on a mesh of n blocks.  FP64: one
+// (20 % faster at every size, 100 to 3000 blocks, than one pair: 24 instead of 12 warps per
+// SM).  FP32, fast build: a pair (one cell is 20 to 100 % slower).  FP32, exact build: one
+// cell where the blocks leave the SMs short of warps.
+template <class T> constexpr int quad_lanes(int n)
+{
+#if BGF_FAST
+    return sizeof(T) == 8 ? 1 : 2;
+#else
+    return sizeof(T) == 8 || n < kOneCellBlocks ? 1 : 2;
+#endif
+}
+
+template <class T, int ENGINE, bool SPLIT, bool POOL, int LANES> cudaError_t configure_quad()
+{
+    constexpr int sm = (int)sizeof(SmemQ<T, LANES>);
+    cudaError_t e = cudaFuncSetAttribute(fluxq_kernel<T, ENGINE, POOL, SPLIT, LANES>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+    if (e != cudaSuccess) return e;
+    return cudaFuncSetAttribute(updateq_kernel<T, ENGINE, POOL, SPLIT, LANES>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
+}
 
 template <class T, int ENGINE, bool SPLIT, bool POOL> cudaError_t configure_one()
 {
@@ -370,35 +392,12 @@ template <class T, int ENGINE, bool SPLIT, bool POOL> cudaError_t configure_one(
     if (e != cudaSuccess) return e;
     e = cudaFuncSetAttribute(update_kernel<T, ENGINE, SPLIT, POOL>, cudaFuncAttributeMaxDynamicSharedMemorySize, sm);
     if (e != cudaSuccess) return e;
-    // two cells per thread
-    e = cudaFuncSetAttribute(flux2_kernel<T, ENGINE, POOL, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)smem2_pred<T>());
-    if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(update2_kernel<T, ENGINE, POOL, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)smem2_corr<T>());
-    if (e != cudaSuccess || SPLIT) return e;  // (the staged layout has no split mode)
-    // staged tiles (persistent CTAs with a producer warp)
-    e = cudaFuncSetAttribute(flux3_kernel<T, ENGINE, POOL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)smem3_pred<T>());
-    if (e != cudaSuccess) return e;
-    return cudaFuncSetAttribute(update3_kernel<T, ENGINE, POOL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)smem3_corr<T>());
-}
-
-// Persistent grid of the staged kernels: CTAs resident on all SMs at once (from the
-// occupancy of the kernel at its shared memory), at most one per block.
-template <class KERN> static int resident_grid(KERN k, size_t smem, int nblk)
-{
-    static int sms = 0;
-    if (sms == 0) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
+    // pairs of cells eight rows apart
+    e = configure_quad<T, ENGINE, SPLIT, POOL, quad_lanes<T>(1 << 30)>();
+    if constexpr (quad_lanes<T>(1 << 30) != quad_lanes<T>(1)) {
+        if (e == cudaSuccess) e = configure_quad<T, ENGINE, SPLIT, POOL, quad_lanes<T>(1)>();
     }
-    int per = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k, NT3, smem) != cudaSuccess || per <= 0) per = 1;
-    const int g = sms * per;
-    return g < nblk ? g : nblk;
+    return e;
 }
 
 template <class T, int ENGINE> cudaError_t configure_engine()
@@ -420,6 +419,41 @@ template <class T> cudaError_t configure_kernels()
     return configure_engine<T, 2>();
 }
 
+// A launch that may start while the kernel before it on the stream still runs (the
+// kernel waits for it itself, pdl_wait): hides the launch, the ramp and the loads that no
+// kernel changes behind the tail of the one before.
+template <class T>
+static void launch_chained(void (*k)(DevModel<T>, StepParams<T>, int), int grid, int nt, size_t smem, cudaStream_t st,
+                           const DevModel<T>& m, const StepParams<T>& p, int parity)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3((unsigned)nt);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = m.pdl ? 1 : 0;
+    (void)cudaLaunchKernelEx(&cfg, k, m, p, parity);  // (an error stays for the caller's cudaGetLastError)
+}
+
+template <class T, bool FLUX, int ENGINE, int LANES>
+static void launch_quad(const DevModel<T>& m, const StepParams<T>& p, int parity, cudaStream_t st, int g, bool pool, bool split)
+{
+    void (*k)(DevModel<T>, StepParams<T>, int);
+    if constexpr (FLUX) k = pool ? fluxq_kernel<T, ENGINE, true, false, LANES> : fluxq_kernel<T, ENGINE, false, false, LANES>;
+    else k = pool ? updateq_kernel<T, ENGINE, true, false, LANES> : updateq_kernel<T, ENGINE, false, false, LANES>;
+    if constexpr (sizeof(T) == 4) {
+        if (split) {
+            if constexpr (FLUX) k = pool ? fluxq_kernel<T, ENGINE, true, true, LANES> : fluxq_kernel<T, ENGINE, false, true, LANES>;
+            else k = pool ? updateq_kernel<T, ENGINE, true, true, LANES> : updateq_kernel<T, ENGINE, false, true, LANES>;
+        }
+    }
+    launch_chained<T>(k, g, Quad<T, LANES>::NT, sizeof(SmemQ<T, LANES>), st, m, p, parity);
+}
+
 // grid: CTAs of the launch (0: one per active block); fewer CTAs loop over the blocks
 template <class T, bool FLUX, int ENGINE>
 static void launch_step_kernel(const DevModel<T>& m, const StepParams<T>& p, int parity, cudaStream_t st, int g)
@@ -428,40 +462,14 @@ static void launch_step_kernel(const DevModel<T>& m, const StepParams<T>& p, int
     const bool pool = m.scen != nullptr;
     bool split = false;
     if constexpr (sizeof(T) == 4) split = m.datum != nullptr;
-    if (!split && m.gen == 3) {
-        // staged tiles, persistent CTAs (the grid argument, when set, is the CTA count)
-        if constexpr (FLUX) {
-            auto k = pool ? flux3_kernel<T, ENGINE, true> : flux3_kernel<T, ENGINE, false>;
-            const int gg = g < m.nblk ? g : resident_grid(k, smem3_pred<T>(), m.nblk);
-            k<<<gg, NT3, smem3_pred<T>(), st>>>(m, p, parity);
-        } else {
-            auto k = pool ? update3_kernel<T, ENGINE, true> : update3_kernel<T, ENGINE, false>;
-            const int gg = g < m.nblk ? g : resident_grid(k, smem3_corr<T>(), m.nblk);
-            k<<<gg, NT3, smem3_corr<T>(), st>>>(m, p, parity);
-        }
-        return;
-    }
     if (m.gen != 1) {
-        // two cells per thread (split precision too; the staged layout falls back here)
-        if constexpr (sizeof(T) == 4) {
-            if (split) {
-                if constexpr (FLUX) {
-                    if (pool) flux2_kernel<T, ENGINE, true, true><<<g, NT2, smem2_pred<T>(), st>>>(m, p, parity);
-                    else flux2_kernel<T, ENGINE, false, true><<<g, NT2, smem2_pred<T>(), st>>>(m, p, parity);
-                } else {
-                    if (pool) update2_kernel<T, ENGINE, true, true><<<g, NT2, smem2_corr<T>(), st>>>(m, p, parity);
-                    else update2_kernel<T, ENGINE, false, true><<<g, NT2, smem2_corr<T>(), st>>>(m, p, parity);
-                }
+        if constexpr (quad_lanes<T>(1 << 30) != quad_lanes<T>(1)) {
+            if (quad_lanes<T>(m.nblk) == quad_lanes<T>(1)) {
+                launch_quad<T, FLUX, ENGINE, quad_lanes<T>(1)>(m, p, parity, st, g, pool, split);
                 return;
             }
         }
-        if constexpr (FLUX) {
-            if (pool) flux2_kernel<T, ENGINE, true><<<g, NT2, smem2_pred<T>(), st>>>(m, p, parity);
-            else flux2_kernel<T, ENGINE, false><<<g, NT2, smem2_pred<T>(), st>>>(m, p, parity);
-        } else {
-            if (pool) update2_kernel<T, ENGINE, true><<<g, NT2, smem2_corr<T>(), st>>>(m, p, parity);
-            else update2_kernel<T, ENGINE, false><<<g, NT2, smem2_corr<T>(), st>>>(m, p, parity);
-        }
+        launch_quad<T, FLUX, ENGINE, quad_lanes<T>(1 << 30)>(m, p, parity, st, g, pool, split);
         return;
     }
     if constexpr (FLUX) {

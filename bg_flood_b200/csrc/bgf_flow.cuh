@@ -131,6 +131,8 @@ template <class T> struct DevModel {
                                       // +-regular_nbx, a domain edge its own block); the two-cell
                                       // kernels then derive ids instead of loading them
     int regular_nby;                  // rows of that grid (nblk / regular_nbx)
+    int pdl;                          // 1: the single-level step kernels are launched as programmatic
+                                      // dependents of the kernel before them (read by the launchers)
     unsigned regular_magic;           // > 0: ib / regular_nbx == umulhi(ib, regular_magic) for every
                                       // block id (checked on the host), else a division
 };

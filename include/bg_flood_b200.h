@@ -206,14 +206,13 @@ int bgf_kernel_timing(bgf_handle* h, double* flux_ms, double* update_ms, int64_t
  * active block; a smaller count makes each CTA loop over blocks (a persistent
  * launch).  Results do not depend on it. */
 int bgf_set_grid(bgf_handle* h, int grid);
-/* Thread layout of the two fused single-level kernels: 2 (default) gives each
- * thread two vertically adjacent cells of a block (128 threads per block, paired
- * FP32 arithmetic in the fast-math build), 1 one cell per thread (256 threads per
- * block), 3 the two-cell arithmetic in persistent CTAs whose fifth warp stages the
- * next block's tile into shared memory with bulk asynchronous copies while the
- * other four compute (the grid then defaults to the CTAs resident on all SMs).
- * The exact build gives the same results bit for bit with each; split-precision
- * handles always use layout 1.  No counterpart in the reference. */
+/* Thread layout of the two fused single-level kernels: 2 (default) works on pairs of
+ * cells eight rows apart -- a pair per thread (128 threads per block, paired FP32
+ * arithmetic in the fast-math build), or one cell of a pair (256 threads) in double
+ * precision and on small meshes of the exact build; 1 is the earlier one cell per
+ * thread; 3 is accepted and runs layout 2 (it was a staged form of it, slower at
+ * every size).  The exact build gives the same results bit for bit with each.  No
+ * counterpart in the reference. */
 int bgf_set_kernel_layout(bgf_handle* h, int cells_per_thread);
 
 /* ------------------------------------------------------------ gauges */
