@@ -162,7 +162,13 @@ struct bgf_handle {
     // multi-level meshes split their active blocks: the chain runs on blocks with a
     // side facing another level, the single-level kernels on the rest ("pure")
     int* d_active_chain = nullptr;
+    int* d_coarse = nullptr;  // chain blocks with a side facing a coarser block, by level
+    std::vector<int> coarse_off;  // offsets of the levels in it (AmrLists)
+    int chain_nofiner = 0, chain_ncoarser = 0;
     int* d_active_pure = nullptr;
+    // the single-level kernels' branch of a multi-level stage, forked from and joined to stream
+    cudaStream_t stream2 = nullptr;
+    cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
     uint8_t* d_nolead = nullptr;  // zeros: the chain's kernels do not write the time slot
     int nchain = 0, npure = 0;
     // refinement pass: bathymetry grid, block origins, flags, children
@@ -911,6 +917,8 @@ static void free_amr(bgf_handle* h)
     dfree(h, h->d_pflag);
     dfree(h, h->d_rank);
     dfree(h, h->d_active_chain);
+    dfree(h, h->d_coarse);
+    h->d_coarse = nullptr;
     dfree(h, h->d_active_pure);
     dfree(h, h->d_nolead);
     h->d_pflag = nullptr;
@@ -949,6 +957,9 @@ int bgf_destroy(bgf_handle* h)
         stage_release(h->tstage[k], h->tstage_bytes[k]);
         if (h->tstage_ev[k]) cudaEventDestroy(h->tstage_ev[k]);
     }
+    if (h->ev_fork) cudaEventDestroy(h->ev_fork);
+    if (h->ev_join) cudaEventDestroy(h->ev_join);
+    if (h->stream2) cudaStreamDestroy(h->stream2);
     if (h->own_stream && h->stream) cudaStreamDestroy(h->stream);
     delete h;
     return BGF_OK;
@@ -961,6 +972,14 @@ static int rebuild_segments(bgf_handle* h);
 static int alloc_amr(bgf_handle* h)
 {
     if (h->d_rank) return BGF_OK;
+    if (!h->stream2) {
+        // (at the priority of the main stream: both branches share the SMs)
+        int prio = 0;
+        if (cudaStreamGetPriority(h->stream, &prio) != cudaSuccess) prio = 0;
+        BGF_CUDA(cudaStreamCreateWithPriority(&h->stream2, cudaStreamNonBlocking, prio));
+        BGF_CUDA(cudaEventCreateWithFlags(&h->ev_fork, cudaEventDisableTiming));
+        BGF_CUDA(cudaEventCreateWithFlags(&h->ev_join, cudaEventDisableTiming));
+    }
     const size_t nb = (size_t)h->nblkmem, es = h->esz;
     bool ok = true;
     for (auto& st : h->d_W)
@@ -970,6 +989,7 @@ static int alloc_amr(bgf_handle* h)
     ok = ok && dalloc(h, (void**)&h->d_pflag, nb * 64) == cudaSuccess;
     ok = ok && dalloc(h, (void**)&h->d_rank, nb * sizeof(int)) == cudaSuccess;
     ok = ok && dalloc(h, (void**)&h->d_active_chain, nb * sizeof(int)) == cudaSuccess;
+    ok = ok && dalloc(h, (void**)&h->d_coarse, nb * sizeof(int)) == cudaSuccess;
     ok = ok && dalloc(h, (void**)&h->d_active_pure, nb * sizeof(int)) == cudaSuccess;
     ok = ok && dalloc(h, (void**)&h->d_nolead, nb) == cudaSuccess;
     if (!ok) {
@@ -1061,6 +1081,30 @@ static int upload_tables(bgf_handle* h)
             for (int k = 0; k < 8; k++) cross = cross || h->level[h->nbr[(size_t)k * nb + ib]] != h->level[ib];
             (cross ? chain : pure).push_back(ib);
         }
+        // the chain's order and its blocks with a coarser side, by level (AmrLists)
+        std::vector<int> kind[3];
+        std::vector<std::vector<int>> by_level(h->maxlev - h->minlev + 1);
+        for (int ib : chain) {
+            bool finer = false, coarser = false;
+            for (int k = 0; k < 8; k++) {
+                const int d = h->level[h->nbr[(size_t)k * nb + ib]] - h->level[ib];
+                finer = finer || d > 0;
+                coarser = coarser || d < 0;
+            }
+            kind[!finer ? 0 : coarser ? 1 : 2].push_back(ib);
+            if (coarser) by_level[h->level[ib] - h->minlev].push_back(ib);
+        }
+        chain.clear();
+        for (auto& k : kind) chain.insert(chain.end(), k.begin(), k.end());
+        h->chain_nofiner = (int)kind[0].size();
+        h->chain_ncoarser = (int)(kind[0].size() + kind[1].size());
+        std::vector<int> coarse;
+        h->coarse_off.assign(1, 0);
+        for (auto& l : by_level) {
+            coarse.insert(coarse.end(), l.begin(), l.end());
+            h->coarse_off.push_back((int)coarse.size());
+        }
+        if (!coarse.empty()) BGF_CUDA(upload(h, h->d_coarse, coarse.data(), sizeof(int) * coarse.size()));
         h->nchain = (int)chain.size();
         h->npure = (int)pure.size();
         if (h->nchain) BGF_CUDA(upload(h, h->d_active_chain, chain.data(), sizeof(int) * h->nchain));
@@ -1639,21 +1683,26 @@ static int enqueue_amr_stage(bgf_handle* h, const DevModel<T>& m, const StepPara
                              bool pool)
 {
     int n = 0;
-    const DevModel<T> mc = chain_model<T>(h, m, pool), mp = pure_model<T>(h, m);
-    if (stage == 0 && h->npure) {
-        if (h->fast) fa::launch_flux<T>(mp, p, h->P.engine, parity, h->stream, 0);
-        else ex::launch_flux<T>(mp, p, h->P.engine, parity, h->stream, 0);
+    const DevModel<T> mc = chain_model<T>(h, m, pool);
+    if (h->npure) {
+        // The two block sets of a stage are independent of one another (the predictor reads
+        // state n, the corrector that and the predictor's tendencies): the single-level kernel
+        // runs beside the chain, which alone leaves most of the SMs waiting on its short
+        // kernels' loads.
+        DevModel<T> mp = pure_model<T>(h, m);
+        mp.pdl = 0;
+        cudaEventRecord(h->ev_fork, h->stream);
+        cudaStreamWaitEvent(h->stream2, h->ev_fork, 0);
+        auto go = stage == 0 ? (h->fast ? fa::launch_flux<T> : ex::launch_flux<T>)
+                             : (h->fast ? fa::launch_update<T> : ex::launch_update<T>);
+        go(mp, p, h->P.engine, parity, h->stream2, 0);
+        cudaEventRecord(h->ev_join, h->stream2);
         n++;
     }
-    n += h->fast ? fa::launch_amr_stage<T>(mc, amr_dev<T>(h), p, h->P.engine, parity, stage, h->minlev, h->maxlev,
-                                          h->stream)
-                 : ex::launch_amr_stage<T>(mc, amr_dev<T>(h), p, h->P.engine, parity, stage, h->minlev, h->maxlev,
-                                          h->stream);
-    if (stage == 1 && h->npure) {
-        if (h->fast) fa::launch_update<T>(mp, p, h->P.engine, parity, h->stream, 0);
-        else ex::launch_update<T>(mp, p, h->P.engine, parity, h->stream, 0);
-        n++;
-    }
+    const AmrLists lists{h->chain_nofiner, h->chain_ncoarser, h->d_coarse, h->coarse_off.data(), h->maxlev - h->minlev + 1};
+    n += h->fast ? fa::launch_amr_stage<T>(mc, amr_dev<T>(h), p, h->P.engine, parity, stage, lists, h->stream)
+                 : ex::launch_amr_stage<T>(mc, amr_dev<T>(h), p, h->P.engine, parity, stage, lists, h->stream);
+    if (h->npure) cudaStreamWaitEvent(h->stream, h->ev_join, 0);
     return n;
 }
 

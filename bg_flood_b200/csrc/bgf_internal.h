@@ -15,6 +15,17 @@ template <class T> struct StepParams;
 template <class T> struct AmrDev;
 template <class T> struct GaugeRingDev;
 
+// Block lists of the multi-level chain.  Its own list (DevModel::active) starts with the
+// blocks without finer neighbours (nofiner of them), then those with finer and coarser ones
+// (up to ncoarser), then the rest.  coarse: the blocks with a side facing a coarser block,
+// coarsest level first (host offsets of the nlev levels, nlev + 1 entries).
+struct AmrLists {
+    int nofiner, ncoarser;
+    const int* coarse;
+    const int* coarse_off;
+    int nlev;
+};
+
 // Gauge sampling after a step (bgf_gauge.cu), built once: it does no arithmetic
 // beyond zs = zb + h.
 template <class T> void launch_gauges(const DevModel<T>& m, const GaugeRingDev<T>& r, int parity, cudaStream_t st);
@@ -36,7 +47,7 @@ template <class T> void launch_gauges(const DevModel<T>& m, const GaugeRingDev<T
     template <class T> cudaError_t configure_amr_kernels();                                                    \
     template <class T>                                                                                         \
     int launch_amr_stage(const DevModel<T>& m, const AmrDev<T>& a, const StepParams<T>& p, int engine,         \
-                         int parity, int stage, int minlev, int maxlev, cudaStream_t st);                      \
+                         int parity, int stage, const AmrLists& lists, cudaStream_t st);                       \
     template <class T> int launch_bed_init(const DevModel<T>& m, const StepParams<T>& p, T* zb, T* gx, T* gy,  \
                                            cudaStream_t st);
 namespace exact {

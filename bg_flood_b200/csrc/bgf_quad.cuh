@@ -974,8 +974,8 @@ template <class T, int LANES, class V>
 __device__ __forceinline__ void reload_faces(SmemQ<T, LANES>& s, const Place<T, LANES>& at, OwnFlux<V>& own)
 {
     const int ox = pfx(at.x, at.r), oy = pfy(at.x, at.r);
-    own.xh = s.fx[0].get(ox, at.l); own.xq = s.fxq().get(ox, at.l);
-    own.yh = s.fy[0].get(oy, at.l); own.yq = s.fyq().get(oy, at.l);
+    own.xh = s.fx[0].get(ox, at.l); own.xq = s.fxq().get(ox, at.l); own.xt = s.fx[2].get(ox, at.l);
+    own.yh = s.fy[0].get(oy, at.l); own.yq = s.fyq().get(oy, at.l); own.yt = s.fy[2].get(oy, at.l);
 }
 
 // updateEVCPU (src/Advection.cu:160-254), Cartesian, for the own cells.
@@ -1122,6 +1122,57 @@ __device__ __forceinline__ T add_rivers_q(const DevModel<T>& m, const StepParams
 {
     return river_cell<T>(m.rivers, m.riv_t, m.riv_q, p.riv_first, p.nriver, calcres<T>(p.delta0, m.level[ib]),
                          p.xo_d + m.bxo[ib], p.yo_d + m.byo[ib], x, y, dh, time);
+}
+
+// Full step of the own cells from state n (AdvkernelCPU with evolv), then friction on the
+// result and rain; the next state goes to buffer nxt.
+template <class T, bool SPLIT, int LANES, class V>
+__device__ __forceinline__ void full_step(const DevModel<T>& m, const StepParams<T>& p, int ib, const Place<T, LANES>& at,
+                                          size_t g, int nxt, T dt, T delta, T D, T rainv, double time, V hold, V uold,
+                                          V vold, V dh, V dhu, V dhv)
+{
+    const bool fm = p.forcemass != 0;
+    const V Dv = cst<V>(D);
+    V ho, uo, vo;
+    if constexpr (SPLIT) advance_split_v<V>(dt, p.eps, fm, Dv, hold, uold, vold, dh, dhu, dhv, ho, uo, vo);
+    else advance_v<V>(dt, p.eps, p.eps_d, fm, hold, uold, vold, dh, dhu, dhv, ho, uo, vo);
+    const V cfv = p.has_cf ? own_of<V>(m.cf, g, 128, at.l) : cst<V>(p.cf);
+    // (split precision: friction on the full depth; the deviation is not changed by it)
+    friction_v<V>(p.frictionmodel, p.g, p.eps, dt, cfv, SPLIT ? add(Dv, ho) : ho, uo, vo);
+    if (p.has_rain) {
+        // AddrainforcingImplicitCPU (src/Updateforcing.cu:530-580): the rain rate at
+        // the start of the step, uniform or gridded
+        V Rainhh;
+        const V mask = m.rainmask ? own_of<V>(m.rainmask, g, 128, at.l) : cst<V>((T)1);
+        if (p.rain_map) {
+            const T xc = (T)p.xo_d + (T)m.bxo[ib] + (T)at.x * delta;
+            auto rate = [&](int y) {
+                return rain_map_at<T>(m.rmap, xc, (T)p.yo_d + (T)m.byo[ib] + (T)y * delta, time);
+            };
+            if constexpr (LANES == 1) Rainhh = rate(at.r + 8 * at.l);
+            else Rainhh = V{rate(at.r), rate(at.r + 8)};
+            const V rr = dv(dv(Rainhh, cst<V>((T)1000.0)), cst<V>((T)3600.0));
+            Rainhh = mul(vmax(mul(rr, cst<V>(dt)), cst<V>((T)0.0)), mask);
+        } else {
+            Rainhh = mul(cst<V>(rainv), mask);  // (the block's uniform depth, above)
+        }
+        const V hi = SPLIT ? add(Dv, ho) : ho;
+        const V qvol = dv(hi, add(hi, Rainhh));
+        ho = add(ho, Rainhh);
+        typename LaneOf<V>::Mask wet;
+        if constexpr (LANES == 1) wet = (double)hi > p.eps_d;
+        else wet = M2{(double)hi.a > p.eps_d, (double)hi.b > p.eps_d};
+        uo = sel(wet, mul(uo, qvol), uo);
+        vo = sel(wet, mul(vo, qvol), vo);
+    }
+    put_own(m.h[nxt], g, at.l, ho);
+    put_own(m.u[nxt], g, at.l, uo);
+    put_own(m.v[nxt], g, at.l, vo);
+    if (m.hmax) {
+        const V hf = SPLIT ? add(Dv, ho) : ho;  // the full depth
+        const V hx = own_of<V>(m.hmax, g, 128, at.l);
+        put_own(m.hmax, g, at.l, sel(gt(hf, hx), hf, hx));
+    }
 }
 
 // Programmatic dependent launch: a step kernel lets the next one start as soon as its own
@@ -1325,48 +1376,8 @@ __device__ __forceinline__ void update_block(SmemQ<T, LANES>& s, const DevModel<
     divergence_q<T, LANES>(s, p, (T)1.0 / ((T)1.0 * delta), at, own, SPLIT ? add(Dv, c[VH]) : c[VH], c[VU], c[VV], dh, dhu,
                            dhv);
     if (p.nriver > 0) dh = rivers(dh);
-    // full step from state n (AdvkernelCPU with evolv), then friction on the result
-    V ho, uo, vo;
-    if constexpr (SPLIT) advance_split_v<V>(dt, p.eps, fm, Dv, hold, uold, vold, dh, dhu, dhv, ho, uo, vo);
-    else advance_v<V>(dt, p.eps, p.eps_d, fm, hold, uold, vold, dh, dhu, dhv, ho, uo, vo);
-    const V cfv = p.has_cf ? own_of<V>(m.cf, g, 128, at.l) : cst<V>(p.cf);
-    // (split precision: friction on the full depth; the deviation is not changed by it)
-    friction_v<V>(p.frictionmodel, p.g, p.eps, dt, cfv, SPLIT ? add(Dv, ho) : ho, uo, vo);
-    if (p.has_rain) {
-        // AddrainforcingImplicitCPU (src/Updateforcing.cu:530-580): the rain rate at
-        // the start of the step, uniform or gridded
-        V Rainhh;
-        const V mask = m.rainmask ? own_of<V>(m.rainmask, g, 128, at.l) : cst<V>((T)1);
-        if (p.rain_map) {
-            const T xc = (T)p.xo_d + (T)m.bxo[ib] + (T)at.x * delta;
-            auto rate = [&](int y) {
-                return rain_map_at<T>(m.rmap, xc, (T)p.yo_d + (T)m.byo[ib] + (T)y * delta, ts.totaltime);
-            };
-            if constexpr (LANES == 1) Rainhh = rate(at.r + 8 * at.l);
-            else Rainhh = V{rate(at.r), rate(at.r + 8)};
-            const V rr = dv(dv(Rainhh, cst<V>((T)1000.0)), cst<V>((T)3600.0));
-            Rainhh = mul(vmax(mul(rr, cst<V>((T)dtd)), cst<V>((T)0.0)), mask);
-        } else {
-            Rainhh = mul(cst<V>(s.rainv), mask);  // (the block's uniform depth, above)
-        }
-        const V hi = SPLIT ? add(Dv, ho) : ho;
-        const V qvol = dv(hi, add(hi, Rainhh));
-        ho = add(ho, Rainhh);
-        typename LaneOf<V>::Mask wet;
-        if constexpr (LANES == 1) wet = (double)hi > p.eps_d;
-        else wet = M2{(double)hi.a > p.eps_d, (double)hi.b > p.eps_d};
-        uo = sel(wet, mul(uo, qvol), uo);
-        vo = sel(wet, mul(vo, qvol), vo);
-    }
     const int nxt = ts.cur ^ 1;
-    put_own(m.h[nxt], g, at.l, ho);
-    put_own(m.u[nxt], g, at.l, uo);
-    put_own(m.v[nxt], g, at.l, vo);
-    if (m.hmax) {
-        const V hf = SPLIT ? add(Dv, ho) : ho;  // the full depth
-        const V hx = own_of<V>(m.hmax, g, 128, at.l);
-        put_own(m.hmax, g, at.l, sel(gt(hf, hx), hf, hx));
-    }
+    full_step<T, SPLIT, LANES>(m, p, ib, at, g, nxt, dt, delta, D, s.rainv, ts.totaltime, hold, uold, vold, dh, dhu, dhv);
     if (lead && tid == 0)
         m.time[2 * sc + (parity ^ 1)] = next_time_state<T>(ts, p, dtd, nxt, m.dtmin + 2 * sc, parity);
 }
