@@ -148,7 +148,7 @@ struct bgf_handle {
     // multi-level meshes: stage tiles with halos, pre-prolongation gradients, face
     // arrays, wet/dry prolongation decisions and the active-list rank of each block
     bool amr = false;
-    int gen = 2;  // single-level stage kernels: 1 one cell per thread, 2 two cells per thread
+    int gen = 2;  // single-level stage kernels: 1 the separate one-cell kernels, 2 the pair kernels
     int minlev = 0, maxlev = 0;
     int steps_launches = 2;  // kernel launches per step
     int grid = 0;            // CTAs of the fused kernels (0: one per block)
@@ -1033,7 +1033,7 @@ static int upload_tables(bgf_handle* h)
         g_last_error = "split precision supports single-level meshes only";
         return BGF_EINVAL;
     }
-    // a full regular grid of blocks in row-major ids: the two-cell kernels derive the
+    // a full regular grid of blocks in row-major ids: the pair kernels derive the
     // ids the tables hold instead of loading them
     h->regular_nbx = 0;
     h->regular_nby = 0;

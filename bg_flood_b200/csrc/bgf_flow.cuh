@@ -124,11 +124,11 @@ template <class T> struct DevModel {
     T* hmax;                          // per cell (256 per block): running maximum depth, or null
     const T* datum;                   // per block slot: datum depth of split mode, or null
     int checklev;                     // fused kernels: verify that neighbours share the block's level
-    int gen;                          // thread layout of the single-level stage kernels: 1 one cell per
-                                      // thread, otherwise two cells per thread (read by the launchers)
+    int gen;                          // thread layout of the single-level stage kernels: 1 the separate
+                                      // one-cell kernels, otherwise the pair kernels (read by the launchers)
     int regular_nbx;                  // > 0: the mesh is a full regular grid of regular_nbx blocks per
                                       // row in row-major ids (active[w] == w, neighbours at +-1 and
-                                      // +-regular_nbx, a domain edge its own block); the two-cell
+                                      // +-regular_nbx, a domain edge its own block); the pair
                                       // kernels then derive ids instead of loading them
     int regular_nby;                  // rows of that grid (nblk / regular_nbx)
     int pdl;                          // 1: the single-level step kernels are launched as programmatic

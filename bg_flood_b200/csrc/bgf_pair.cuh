@@ -1,6 +1,5 @@
-// Two cells per thread.  The second-generation single-level stage kernels
-// (bgf_flow2.cuh) give each thread two vertically adjacent cells and evaluate
-// both with one instruction stream: a value of the pair type V2<T> holds the two
+// Two cells per thread.  The stage kernels of bgf_quad.cuh give each thread two
+// cells of a column eight rows apart and evaluate both with one instruction stream: a value of the pair type V2<T> holds the two
 // cells' values.  For FP32 in the fast build the pair is one 64-bit register and
 // additions, subtractions, products and fused multiply-adds use the paired FP32
 // instructions of sm_100 (add / sub / mul / fma .f32x2, PTX ISA 8.6): one issue

@@ -38,7 +38,7 @@
 // Measured against the kernels this replaced (pairs of adjacent rows, faces from gradients)
 // on B200: 545 -> 477 thread-instructions per cell in the predictor and 633 -> 579 in the
 // corrector (fast FP32); with the chained launches (pdl_trigger) the step of the 1024x1024
-// run-up takes 49.8 instead of 56.6 us, of a 4096x4096 one 705 instead of 769 us.  Two
+// run-up takes 48.9 instead of 56.6 us, of a 4096x4096 one 692 instead of 769 us.  Two
 // pairs per thread (398 and 503 instructions per cell, 128 registers) ran as fast on large
 // grids and slower on all others; one warp marching over a block's rows (no barriers) was
 // half as fast, its warps out of step in the instruction cache.
@@ -540,7 +540,7 @@ __device__ __forceinline__ void ring_cell(const DevModel<T>& m, int ib, int k, i
 }
 
 // Whether the slopes of the ring are spread over threads 0..127 (two a ring cell) instead of
-// made by one pass of a warp (two warps for LANES = 1): the exact build's are long enough to
+// made by two warps: the exact build's are long enough to
 // keep the other warps waiting (12,288 blocks: 426 instead of 453 us per step), the fast
 // build's are not (146 instead of 142 us).
 template <class T, int LANES> struct RingPass {
@@ -561,8 +561,8 @@ template <class T, int LANES> struct Place {
         constexpr int NW = Quad<T, LANES>::NW;
         const int hsh = (int)(((unsigned)w * 0x9E3779B1u) >> 30);
         const int at = ((tid_ >> 5) + hsh) & (NW - 1);
-        ring = LANES == 2 ? at == 0 : at == 0 || at == 4;
-        rl = at >> 2;
+        ring = at == 0 || at == (LANES == 2 ? 1 : 4);
+        rl = at != 0;
         extra = at == 2;
     }
 };
@@ -570,8 +570,8 @@ template <class T, int LANES> struct Place {
 // Bed gradients the engine-1 wet-slope reset reads: the own ones and those of the thread's
 // ring cells (spread: towards the block).
 template <class T, int LANES> struct BedGradQ {
-    using V = typename ValOf<T, LANES>::V;
-    V gx, gy, ring;
+    typename ValOf<T, LANES>::V gx, gy;
+    T ring;
 };
 template <class T, int ENGINE, int LANES>
 __device__ __forceinline__ void load_bedgrad_q(const DevModel<T>& m, int ib, const Place<T, LANES>& at, BedGradQ<T, LANES>& b)
@@ -586,11 +586,11 @@ __device__ __forceinline__ void load_bedgrad_q(const DevModel<T>& m, int ib, con
         if constexpr (RingPass<T, LANES>::spread) {
             const int side = at.tid >> 5, t = (at.tid >> 1) & 15;
             const T q = side < 2 ? bx[hi18(side ? BW : -1, t)] : by[hi18(t, side == 3 ? BW : -1)];
-            b.ring = cst<V>(side & 1 ? -q : q);
+            b.ring = side & 1 ? -q : q;
         } else if (at.ring) {
             const int l = at.tid & 31;
             const T* p = l < 16 ? bx + hi18(l < 8 ? -1 : BW, l & 7) : by + hi18(l & 15, -1);
-            b.ring = own_of<V>(p, 0, l < 16 ? 8 * 18 : 17 * 18, at.rl);
+            b.ring = p[at.rl ? (l < 16 ? 8 : 17) * 18 : 0];
         }
     }
 }
@@ -755,7 +755,7 @@ __device__ __forceinline__ T tile_faces(SmemQ<T, LANES>& s, const StepParams<T>&
             const T Hr = SPLIT ? D + n0 : n0;
             T c1 = hd_s;
             if (part == 0) {
-                g1 = wetslope_q<T>(hd_s, n1, Hr, f1, i1, g1, g0, lane_of(bg.ring, 0));
+                g1 = wetslope_q<T>(hd_s, n1, Hr, f1, i1, g1, g0, bg.ring);
                 // the velocities' factor (both_sides)
                 const T q = dv(mul(hd_s, g0), Hr);
 #if BGF_FAST
@@ -782,59 +782,45 @@ __device__ __forceinline__ T tile_faces(SmemQ<T, LANES>& s, const StepParams<T>&
         q[0] = o0;
         q[nq] = o1;
     }
-    // ---- the ring: lanes 0..7 the column -1, 8..15 the column 16 (pairs of rows), lanes
-    // 16..31 the cells at rows -1 and 16 of a column.  The inward side only.
+    // ---- the ring in two warps (rl): lanes 0..7 the column -1, 8..15 the column 16 (rows
+    // 0..7 and 8..15), lanes 16..31 the rows -1 and 16.  The inward side only.
     if (!RingPass<T, LANES>::spread && at.ring) {
         const bool isx = lane < 16;
-        // tile index of the two cells, step across the side
-        const int pa = isx ? pt(lane < 8 ? -1 : BW, lane & 7) : pt(lane & 15, -1), pb = isx ? pa : pt(lane & 15, 8);
-        const int ia = LANES == 2 ? 2 * pa : at.rl ? 240 + pb : pa, ib2 = LANES == 2 ? 2 * pb + 1 : ia;
+        // tile index of the cell, step across the side
+        const int pa = pt(isx ? (lane < 8 ? -1 : BW) : lane & 15, isx ? lane & 7 : at.rl ? 8 : -1);
+        const int ia = LANES == 2 ? 2 * pa + at.rl : 240 * at.rl + pa;
         const int d = (isx ? 1 : 20) * LANES;
         const int iu = isx ? VU : VV, iv = isx ? VV : VU;
-        const T sa = isx && lane >= 8 ? -hd_s : hd_s, sb = lane < 8 ? hd_s : -hd_s;
-        const V sg = lanes_of<V>(sa, sb, at.rl);
-        V q0[4], gr[4], zm, zp;
+        const T sg = (isx ? lane >= 8 : at.rl != 0) ? -hd_s : hd_s;
+        T q0[4], gr[4], zm, zp;
 #pragma unroll
         for (int j = 0; j < 4; j++) {
-            const T* a = s.t[j == 0 ? VH : j == 1 ? VZS : j == 2 ? iu : iv].a;
-            auto at2 = [&](int k) {
-                if constexpr (LANES == 1) return a[ia + k];
-                else return V{a[ia + k], a[ib2 + k]};
-            };
-            const V m0 = at2(-d), p0 = at2(d);
-            q0[j] = at2(0);
-            gr[j] = slope_q<V>(th, thr, hr, m0, q0[j], p0, delta, rdelta);
+            const T* a = s.t[j == 0 ? VH : j == 1 ? VZS : j == 2 ? iu : iv].a + ia;
+            const T m0 = a[-d], p0 = a[d];
+            q0[j] = a[0];
+            gr[j] = slope_q<T>(p.theta, thr_s, hr_s, m0, q0[j], p0, delta, rdelta);
             if (j == 1) { zm = m0; zp = p0; }
         }
-        const V Hr = full(q0[0]);
-        if constexpr (ENGINE == 1) gr[1] = wetslope_q<V>(dx, q0[1], Hr, zm, zp, gr[1], gr[0], bg.ring);
-        SideQ<V> in, outw;
+        const T Hr = SPLIT ? D + q0[0] : q0[0];
+        if constexpr (ENGINE == 1) gr[1] = wetslope_q<T>(hd_s, q0[1], Hr, zm, zp, gr[1], gr[0], bg.ring);
+        SideQ<T> in, outw;
         // (both_sides with the signed half spacing: its high side is the inward one)
-        both_sides<V, ENGINE>(sg, q0[0], q0[1], q0[2], q0[3], gr[0], gr[1], gr[2], gr[3], Hr, eps, outw, in);
-        if constexpr (LANES == 2) {
-            T *da, *db;
-            int na, nb;  // steps between the values' arrays
-            if (lane < 8) { da = s.nx[0].a + 2 * pnx(-1, lane); db = da + 1; na = nb = 272; }
-            else if (lane < 16) { da = s.ex[0].a + 2 * (lane - 8); db = da + 1; na = nb = 16; }
-            else { da = s.ny[0].a + 2 * pny(lane - 16, -1); db = s.ey[0] + lane - 16; na = 288; nb = 16; }
-            da[0] = in.h.a; da[na] = in.e.a; da[2 * na] = in.n.a; da[3 * na] = in.t.a;
-            db[0] = in.h.b; db[nb] = in.e.b; db[2 * nb] = in.n.b; db[3 * nb] = in.t.b;
-        } else {
-            T* da;
-            int na;
-            if (lane < 8) { da = s.nx[0].a + 136 * at.rl + pnx(-1, lane); na = 272; }
-            else if (lane < 16) { da = s.ex[0].a + 8 * at.rl + lane - 8; na = 16; }
-            else if (at.rl == 0) { da = s.ny[0].a + pny(lane - 16, -1); na = 288; }
-            else { da = s.ey[0] + lane - 16; na = 16; }
-            da[0] = in.h; da[na] = in.e; da[2 * na] = in.n; da[3 * na] = in.t;
-        }
+        both_sides<T, ENGINE>(sg, q0[0], q0[1], q0[2], q0[3], gr[0], gr[1], gr[2], gr[3], Hr, p.epsface, outw, in);
+        T* da;
+        int na;  // step between the values' arrays
+        if (lane < 8) { da = &s.nx[0].cell(pnx(-1, lane), at.rl); na = 272; }
+        else if (lane < 16) { da = &s.ex[0].cell(lane - 8, at.rl); na = 16; }
+        else if (at.rl == 0) { da = &s.ny[0].cell(pny(lane - 16, -1), 0); na = 288; }
+        else { da = s.ey[0] + lane - 16; na = 16; }
+        da[0] = in.h; da[na] = in.e; da[2 * na] = in.n; da[3 * na] = in.t;
     }
     __syncthreads();
     // ---- faces
-    const V g = cst<V>(p.g), epsi = cst<V>(p.epsi), ga = cst<V>(p.g * (T)0.5);
-    auto face = [&](const FaceQ<V>& f) {
-        if constexpr (SPLIT) return face_q_split<V, ENGINE>(f, Dv, g, ga, epsi, eps);
-        else return face_q<V, ENGINE>(f, g, ga, epsi, eps);
+    auto face = [&](const auto& f) {
+        using F = std::remove_cv_t<decltype(f.hi)>;
+        const F g = cst<F>(p.g), ga = cst<F>(p.g * (T)0.5), epsi = cst<F>(p.epsi), ef = cst<F>(p.epsface);
+        if constexpr (SPLIT) return face_q_split<F, ENGINE>(f, cst<F>(D), g, ga, epsi, ef);
+        else return face_q<F, ENGINE>(f, g, ga, epsi, ef);
     };
     V ax;
     // (source-term beds: engine 1 the bed, engine 2 the surface less the depth)
@@ -905,65 +891,52 @@ __device__ __forceinline__ T tile_faces(SmemQ<T, LANES>& s, const StepParams<T>&
         if constexpr (SPEED) amax = sel(q.wet, vmax(ax, q.a), cst<V>((T)0));
     }
     // the faces on the right column (pairs of rows) and the top row (pairs of columns)
-    if (at.extra && (LANES == 1 || lane < 16)) {
+    // (one face a lane: with a pair in each of half the lanes the other warps wait longer,
+    // 428 instead of 408 us per step for 12,288 blocks of the exact build, 152 instead of
+    // 147 us in split precision)
+    if (at.extra) {
         const bool isx = (lane & 15) < 8;
-        const int q = lane & 7, el = lane >> 4;  // (one cell per thread: the second of the two cells)
+        const int q = lane & 7, el = lane >> 4;  // (which of the two cells)
         // the two cells: rows q and q + 8 of the column 16, or row 16 of the columns 2q, 2q + 1
         const int i0 = isx ? pt(BW, q) : pt(2 * q, 8), z0 = isx ? pz(BW, q) : pz(2 * q, 8);
         const int n0 = isx ? pnx(BW - 1, q) : pny(2 * q, 7), nst = isx ? 272 : 288;
         const T *nn = isx ? s.nx[0].a : s.ny[0].a, *ei = isx ? s.ex[0].a : s.ey[0];
         const int d = (isx ? 1 : 20) * LANES, dz = (isx ? 1 : 18) * LANES;
-        // element of the first cell, and step to the second, in an array of n pairs
+        // element of the cell in an array of n pairs
         auto first = [&](int pr, int n) {
-            if constexpr (LANES == 2) return 2 * pr + (isx ? 0 : 1);
+            if constexpr (LANES == 2) return 2 * pr + (isx ? el : 1 + 2 * el);
             else return isx ? pr + el * n : pr + el + n;
         };
-        const int step = isx ? 1 : 2;
-        auto two = [&](const T* a, int k) {
-            if constexpr (LANES == 1) return a[k];
-            else return V{a[k], a[k + step]};
-        };
         const int ti_ = first(i0, 240), zi_ = first(z0, 180), ni = first(n0, nst / 2);
-        const int ii = LANES == 2 ? 2 * q : isx ? q + 8 * el : 2 * q + el;
-        auto low = [&](int v) {
-            if constexpr (LANES == 1) return ei[16 * v + ii];
-            else return V{ei[16 * v + ii], ei[16 * v + ii + 1]};
-        };
-        FaceQ<V> f;
+        const int ii = LANES == 1 && isx ? q + 8 * el : 2 * q + el;
+        auto low = [&](int v) { return ei[16 * v + ii]; };
+        FaceQ<T> f;
         f.hI = low(0); f.eI = low(1); f.nI = low(2); f.tI = low(3);
-        f.hN = two(nn, ni); f.eN = two(nn + nst, ni); f.nN = two(nn + 2 * nst, ni); f.tN = two(nn + 3 * nst, ni);
-        f.hi = f.hsi = two(s.t[VH].a, ti_);
-        f.hn = f.hsn = two(s.t[VH].a, ti_ - d);
+        f.hN = nn[ni]; f.eN = nn[ni + nst]; f.nN = nn[ni + 2 * nst]; f.tN = nn[ni + 3 * nst];
+        f.hi = f.hsi = s.t[VH].a[ti_];
+        f.hn = f.hsn = s.t[VH].a[ti_ - d];
         if constexpr (ENGINE == 1) {
-            f.zri = two(s.zb.a, zi_);
-            f.zrn = two(s.zb.a, zi_ - dz);
+            f.zri = s.zb.a[zi_];
+            f.zrn = s.zb.a[zi_ - dz];
         } else {
-            f.zri = sub(two(s.t[VZS].a, ti_), f.hi);
-            f.zrn = sub(two(s.t[VZS].a, ti_ - d), f.hn);
+            f.zri = sub(s.t[VZS].a[ti_], f.hi);
+            f.zrn = sub(s.t[VZS].a[ti_ - d], f.hn);
         }
         if constexpr (SUB) {
             const int sd = isx ? 1 : 3;
             const int j0 = isx ? q : 2 * q, j1 = isx ? q + 8 : 2 * q + 1;
             if (subf->on[sd]) {
-                f.hsi = lanes_of<V>(subf->h[sd][j0], subf->h[sd][j1], el);
-                f.zri = lanes_of<V>(subf->z[sd][j0], subf->z[sd][j1], el);
+                f.hsi = lanes_of<T>(subf->h[sd][j0], subf->h[sd][j1], el);
+                f.zri = lanes_of<T>(subf->z[sd][j0], subf->z[sd][j1], el);
             }
         }
-        const FluxQ<V> w = face(f);
+        const FluxQ<T> w = face(f);
         T *o0 = isx ? s.fx[0].a : s.fy[0].a, *oq = isx ? s.fxq().a : s.fyq().a;
         const int fo = first(isx ? pfx(BW, q) : pfy(2 * q, 8), nst / 2), fq = first(isx ? pfx(BW, q) : pfy(2 * q, 8), 240);
-        auto put2 = [&](T* a, int k, V v) {
-            if constexpr (LANES == 1) {
-                a[k] = v;
-            } else {
-                a[k] = v.a;
-                a[k + step] = v.b;
-            }
-        };
-        put2(o0, fo, w.Fh);
-        put2(o0 + nst, fo, w.S);
-        put2(o0 + 2 * nst, fo, w.Ft);
-        if (allfaces) put2(oq, fq, w.Fq);
+        o0[fo] = w.Fh;
+        o0[fo + nst] = w.S;
+        o0[fo + 2 * nst] = w.Ft;
+        if (allfaces) oq[fq] = w.Fq;
     }
     if constexpr (LANES == 1) return amax;
     else return amax.a > amax.b ? amax.a : amax.b;
