@@ -96,6 +96,17 @@ __device__ __forceinline__ float rcpa(float y)
     asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(y));
     return r;
 }
+// Single lanes with one choice of what is fused (an expression leaves it to the compiler, which
+// may take the other of two products): mad always, operands of *_apart never.
+__device__ __forceinline__ float mad(float x, float y, float z) { return __fmaf_rn(x, y, z); }
+__device__ __forceinline__ double mad(double x, double y, double z) { return __fma_rn(x, y, z); }
+__device__ __forceinline__ float sub_apart(float x, float y) { return __fsub_rn(x, y); }
+__device__ __forceinline__ V2<float> sub_apart(V2<float> x, V2<float> y) { return sub(x, y); }
+__device__ __forceinline__ float mul_apart(float x, float y) { return __fmul_rn(x, y); }
+__device__ __forceinline__ double mul_apart(double x, double y) { return __dmul_rn(x, y); }
+__device__ __forceinline__ double add_apart(double x, double y) { return __dadd_rn(x, y); }
+__device__ __forceinline__ float rcp_v(float y) { return rcpa(y); }
+__device__ __forceinline__ V2<float> rcp_v(V2<float> y) { return V2<float>{rcpa(y.a), rcpa(y.b)}; }
 __device__ __forceinline__ float dv(float x, float y) { return x * rcpa(y); }
 __device__ __forceinline__ V2<float> dv(V2<float> x, V2<float> y) { return mul(x, V2<float>{rcpa(y.a), rcpa(y.b)}); }
 // Cube root for Manning's friction factor: h^(1/3) = 2^(log2(h) / 3) with the
@@ -114,6 +125,7 @@ __device__ __forceinline__ V2<float> add(V2<float> x, V2<float> y) { return V2<f
 __device__ __forceinline__ V2<float> sub(V2<float> x, V2<float> y) { return V2<float>{__fsub_rn(x.a, y.a), __fsub_rn(x.b, y.b)}; }
 __device__ __forceinline__ V2<float> mul(V2<float> x, V2<float> y) { return V2<float>{__fmul_rn(x.a, y.a), __fmul_rn(x.b, y.b)}; }
 __device__ __forceinline__ V2<float> mad(V2<float> x, V2<float> y, V2<float> z) { return add(mul(x, y), z); }
+template <class V> __device__ __forceinline__ V sub_apart(V x, V y) { return sub(x, y); }
 #endif
 
 // ---------------------------------------------------------------- FP64 pairs

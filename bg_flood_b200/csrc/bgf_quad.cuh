@@ -38,7 +38,7 @@
 // Measured against the kernels this replaced (pairs of adjacent rows, faces from gradients)
 // on B200: 545 -> 477 thread-instructions per cell in the predictor and 633 -> 579 in the
 // corrector (fast FP32); with the chained launches (pdl_trigger) the step of the 1024x1024
-// run-up takes 48.9 instead of 56.6 us, of a 4096x4096 one 692 instead of 769 us.  Two
+// run-up takes 51.9 instead of 56.6 us, of a 4096x4096 one 729 instead of 769 us.  Two
 // pairs per thread (398 and 503 instructions per cell, 128 registers) ran as fast on large
 // grids and slower on all others; one warp marching over a block's rows (no barriers) was
 // half as fast, its warps out of step in the instruction cache.
@@ -157,7 +157,14 @@ template <class V> __device__ __forceinline__ V minmod_v(V theta, V s0, V s1, V 
 
 // x / delta for the block spacing (div_by): the fast build multiplies by the rounded
 // reciprocal, the exact build takes Markstein's correctly rounded quotient.
-template <class T> __device__ __forceinline__ T divd_v(T x, T d, T r) { return div_by<T>(x, d, r); }
+template <class T> __device__ __forceinline__ T divd_v(T x, T d, T r)
+{
+#if BGF_FAST
+    return mul_apart(x, r);
+#else
+    return div_by<T>(x, d, r);
+#endif
+}
 template <class T> __device__ __forceinline__ V2<T> divd_v(V2<T> x, T d, T r)
 {
 #if BGF_FAST
@@ -178,11 +185,12 @@ __device__ __forceinline__ float xmin(float x, float y)
 __device__ __forceinline__ V2<float> xmin(V2<float> x, V2<float> y) { return V2<float>{xmin(x.a, y.a), xmin(x.b, y.b)}; }
 #endif
 
-// Limited slope minmod2(theta, s0, s1, s2) / delta.  Fast FP32 build: the smaller
-// one-sided difference, positive when both have one sign and cut to zero otherwise,
-// scaled by theta / delta; then the smaller magnitude of it and half the central
-// difference over delta, which gives the sign (three min / max per lane, the value of
-// the selecting form).
+// Limited slope minmod2(theta, s0, s1, s2) / delta.  Fast FP32 build: s0 < s1 < s2 (or
+// s0 > s1 > s2) holds exactly when the product of the one-sided differences is positive (a
+// product flushed to zero only drops a slope below 1e-19); the result is then the smaller
+// magnitude of theta / delta times the smaller difference and half the central difference
+// over delta, with the sign of the latter.  (The bits of the form with three candidates:
+// rounding is monotonic.)
 template <class V>
 __device__ __forceinline__ V slope_q(V th, V thr, V hr, V s0, V s1, V s2, typename LaneOf<V>::T delta,
                                      typename LaneOf<V>::T rdelta)
@@ -190,7 +198,8 @@ __device__ __forceinline__ V slope_q(V th, V thr, V hr, V s0, V s1, V s2, typena
     using T = typename LaneOf<V>::T;
 #if BGF_FAST
     if constexpr (sizeof(T) == 4) {
-        const V p = vmax(xmin(sub(s1, s0), sub(s2, s1)), cst<V>((T)0.0));
+        const V a = sub(s1, s0), b = sub(s2, s1), zero = cst<V>((T)0.0);
+        const V p = sel(gt(mul(a, b), zero), xmin(a, b), zero);
         return xmin(mul(thr, p), mul(hr, sub(s2, s0)));
     }
 #endif
@@ -212,22 +221,6 @@ __device__ __forceinline__ V wetslope_v(V hdelta, V zsi, V hi, V zsm, V zsp, V d
     return sel(reset, add(dh, dzb), dzs);
 }
 
-// Wet-slope reset (wetslope); the fast build compares magnitudes instead of squares.
-template <class V>
-__device__ __forceinline__ V wetslope_q(V hdelta, V zsi, V hi, V zsm, V zsp, V dzs, V dh, V dzb)
-{
-#if BGF_FAST
-    using T = typename LaneOf<V>::T;
-    if constexpr (sizeof(T) == 4) {
-        const V base = sub(zsi, hi);
-        const V e = mul(hdelta, sub(dzs, dh));
-        const auto reset = gt(vabs(dzs), vabs(dzb)) && (gt(sub(base, e), zsm) || gt(add(base, e), zsp));
-        return sel(reset, add(dh, dzb), dzs);
-    }
-#endif
-    return wetslope_v<V>(hdelta, zsi, hi, zsm, zsp, dzs, dh, dzb);
-}
-
 // A face between cell n (low side) and cell i: the states reconstructed on it (depth,
 // surface (engine 2: bed), normal and tangential velocity), the cells' own depths and the
 // depth and bed of the source terms (the cells' own, or a coarser cell's at its face).
@@ -241,12 +234,17 @@ template <class V> struct FluxQ {
     typename LaneOf<V>::Mask wet;
 };
 
-// face_flux (bgf_numerics.cuh) from the reconstructed states.
+// face_flux (bgf_numerics.cuh) from the reconstructed states.  Wherever a product feeds a
+// sum it is written as mad: the fast build fuses the two, and left to itself the compiler
+// does not choose the same product in the scalar and in the paired form.  A face that one
+// block solves as a scalar (the right column and the top row) is half of a pair on its
+// neighbour, and has to come out the same on both (mass is conserved to rounding then).
 template <class V, int ENGINE>
 __device__ __forceinline__ FluxQ<V> face_q(const FaceQ<V>& f, V g, V ga, V epsi, V eps)
 {
     using T = typename LaneOf<V>::T;
     const V zero = cst<V>((T)0.0), half = cst<V>((T)0.5), two = cst<V>((T)2.0), mone = cst<V>((T)-1.0);
+    const V nga = mul(mone, ga);
     FluxQ<V> r;
     r.wet = gt(f.hi, eps) || gt(f.hn, eps);
     V fh, fu, ft, fq, s, a;
@@ -263,18 +261,18 @@ __device__ __forceinline__ FluxQ<V> face_q(const FaceQ<V>& f, V g, V ga, V epsi,
         const auto live = gt(a, epsi);
         const V ad = dv(cst<V>((T)1.0), sub(ap, am));
         const V qm = mul(hm, um), qp = mul(hp, up), apm = mul(ap, am);
-        const V fhl = mul(mad(apm, sub(hp, hm), sub(mul(ap, qm), mul(am, qp))), ad);
+        const V nam = mul(mone, am);
+        const V fhl = mul(mad(apm, sub(hp, hm), mad(ap, qm, mul(nam, qp))), ad);
         const V ful = mul(mad(apm, sub(qp, qm),
-                              sub(mul(ap, mad(qm, um, mul(ga, mul(hm, hm)))), mul(am, mad(qp, up, mul(ga, mul(hp, hp)))))),
+                              mad(ap, mad(qm, um, mul(ga, mul(hm, hm))), mul(nam, mad(qp, up, mul(ga, mul(hp, hp)))))),
                           ad);
         fh = sel(live, fhl, zero);
         fu = sel(live, ful, zero);
         a = sel(live, a, zero);
         ft = mul(sel(gt(fh, zero), f.tN, f.tI), fh);
-        const V sl = mul(ga, mad(add(f.hI, f.hsi), sub(f.zri, f.eI), sub(mul(hp, hp), mul(f.hI, f.hI))));
-        const V sr = mul(ga, mad(add(f.hN, f.hsn), sub(f.zrn, f.eN), sub(mul(hm, hm), mul(f.hN, f.hN))));
-        fq = sub(fu, sl);
-        s = sub(fu, sr);
+        const V nhI = mul(mone, f.hI), nhN = mul(mone, f.hN);
+        fq = mad(nga, mad(add(f.hI, f.hsi), sub(f.zri, f.eI), mad(nhI, f.hI, mul(hp, hp))), fu);
+        s = mad(nga, mad(add(f.hN, f.hsn), sub(f.zrn, f.eN), mad(nhN, f.hN, mul(hm, hm))), fu);
     } else {
         const V zA = vmax(sub(f.eI, f.hI), sub(f.eN, f.hN));
         const V zCN = vmin(zA, vmin(f.eN, f.eI));
@@ -284,50 +282,38 @@ __device__ __forceinline__ FluxQ<V> face_q(const FaceQ<V>& f, V g, V ga, V epsi,
         const V cm = vsqrt(mul(g, hm)), cp = vsqrt(mul(g, hp));
         const V fhm = mul(um, hm), fhp = mul(up, hp);
         // hllc (src/Reimann.cu:838-877)
+        const V ustar = sub(mad(add(um, up), half, cm), cp);
+        const V cstar = mad(add(cm, cp), half, mul(sub(um, up), cst<V>((T)0.25)));
+        const V SL = sel(eq(hm, zero), mad(cst<V>((T)-2.0), cp, up), vmin(sub(um, cm), sub(ustar, cstar)));
+        const V SR = sel(eq(hp, zero), mad(two, cm, um), vmax(add(up, cp), add(ustar, cstar)));
+        const V fum = mul(hm, mad(um, um, mul(mul(g, hm), half)));
+        const V fup = mul(hp, mad(up, up, mul(mul(g, hp), half)));
+        const V SLSR = mul(SL, SR);
+        const V den = sub(SR, SL);
+        const V nSL = mul(mone, SL);
+        const V nh = mad(SLSR, sub(hp, hm), mad(nSL, fhp, mul(SR, fhm)));
+        const V nq = mad(SLSR, mad(hp, up, mul(mone, fhm)), mad(nSL, fup, mul(SR, fum)));
+        V fhM, fqM;
 #if BGF_FAST
         if constexpr (sizeof(T) == 4) {
-            // With the Riemann invariants A = um + 2 cm and B = up - 2 cp the star values are
-            // u* - c* = (A + 3 B) / 4 and u* + c* = (3 A + B) / 4, and A and B are also the
-            // speeds next to a dry side.  The star fluxes with the speeds cut at zero are the
-            // supersonic ones too; the cut of SR at a tiny speed keeps the quotient finite
-            // where both speeds are zero.
-            const V A = mad(two, cm, um), B = mad(cst<V>((T)-2.0), cp, up);
-            const V q = cst<V>((T)0.25), tq = cst<V>((T)0.75);
-            const V SL = sel(eq(hm, zero), B, vmin(sub(um, cm), mad(tq, B, mul(q, A))));
-            const V SR = sel(eq(hp, zero), A, vmax(add(up, cp), mad(tq, A, mul(q, B))));
-            a = vmax(vabs(SL), vabs(SR));
-            const V L = vmin(SL, zero), R = vmax(SR, cst<V>((T)1e-30));
-            const V nL = mul(mone, L), LR = mul(L, R);
-            const V rd = dv(cst<V>((T)1.0), add(R, nL));
-            const V fum = mad(fhm, um, mul(mul(ga, hm), hm)), fup = mad(fhp, up, mul(mul(ga, hp), hp));
-            fh = mul(mad(LR, sub(hp, hm), mad(nL, fhp, mul(R, fhm))), rd);
-            fu = mul(mad(LR, sub(fhp, fhm), mad(nL, fup, mul(R, fum))), rd);
-            ft = mul(sel(gt(fh, zero), f.tN, f.tI), fh);
-            fq = mad(mul(ga, add(f.hsi, hp)), sub(zCN, f.zri), fu);
-            s = mad(mul(ga, add(hm, f.hsn)), sub(zCN, f.zrn), fu);
+            // one reciprocal of the wave-speed spread for both star-region fluxes
+            const V rden = rcp_v(den);
+            fhM = mul(nh, rden);
+            fqM = mul(nq, rden);
         } else
 #endif
         {
-            const V ustar = sub(mad(add(um, up), half, cm), cp);
-            const V cstar = mad(add(cm, cp), half, mul(sub(um, up), cst<V>((T)0.25)));
-            const V SL = sel(eq(hm, zero), mad(cst<V>((T)-2.0), cp, up), vmin(sub(um, cm), sub(ustar, cstar)));
-            const V SR = sel(eq(hp, zero), mad(two, cm, um), vmax(add(up, cp), add(ustar, cstar)));
-            const V fum = mul(hm, mad(um, um, mul(mul(g, hm), half)));
-            const V fup = mul(hp, mad(up, up, mul(mul(g, hp), half)));
-            const V SLSR = mul(SL, SR);
-            const V den = sub(SR, SL);
-            const V nSL = mul(mone, SL);
-            const V fhM = dv(mad(SLSR, sub(hp, hm), mad(nSL, fhp, mul(SR, fhm))), den);
-            const V fqM = dv(mad(SLSR, sub(fhp, fhm), mad(nSL, fup, mul(SR, fum))), den);
-            const auto caseL = le(zero, SL);
-            const auto caseR = ge(zero, SR);
-            fh = sel(caseL, fhm, sel(caseR, fhp, fhM));
-            fu = sel(caseL, fum, sel(caseR, fup, fqM));
-            a = vmax(vabs(SL), vabs(SR));
-            ft = mul(sel(gt(fh, zero), f.tN, f.tI), fh);
-            fq = sub(fu, mul(mul(ga, add(f.hsi, hp)), sub(f.zri, zCN)));
-            s = sub(fu, mul(mul(ga, add(hm, f.hsn)), sub(f.zrn, zCN)));
+            fhM = dv(nh, den);
+            fqM = dv(nq, den);
         }
+        const auto caseL = le(zero, SL);
+        const auto caseR = ge(zero, SR);
+        fh = sel(caseL, fhm, sel(caseR, fhp, fhM));
+        fu = sel(caseL, fum, sel(caseR, fup, fqM));
+        a = vmax(vabs(SL), vabs(SR));
+        ft = mul(sel(gt(fh, zero), f.tN, f.tI), fh);
+        fq = mad(mul(nga, add(f.hsi, hp)), sub(f.zri, zCN), fu);
+        s = mad(mul(nga, add(hm, f.hsn)), sub(f.zrn, zCN), fu);
     }
     r.Fh = sel(r.wet, fh, zero);
     r.Fq = sel(r.wet, fq, zero);
@@ -346,12 +332,12 @@ __device__ __forceinline__ FluxQ<V> face_q_split(const FaceQ<V>& f, V D, V g, V 
     using T = typename LaneOf<V>::T;
     const V zero = cst<V>((T)0.0), one = cst<V>((T)1.0), two = cst<V>((T)2.0), mone = cst<V>((T)-1.0);
     const V half = cst<V>((T)0.5), quarter = cst<V>((T)0.25);
-    const V nD = mul(mone, D);
-    const V shift = mul(mul(mul(mone, ga), D), D);  // -ga * D * D
+    const V nD = mul(mone, D), nga = mul(mone, ga);
+    const V shift = mul(mul(nga, D), D);  // -ga * D * D
     FluxQ<V> r;
     const V Hi = add(D, f.hi), Hn = add(D, f.hn);  // full depths
     r.wet = gt(Hi, eps) || gt(Hn, eps);
-    V fh, fu, ft, sl, sr, a;
+    V fh, fu, ft, fq, s, a;
     if constexpr (ENGINE == 2) {
         const V zlr = vmax(f.eI, f.eN);
         const V up = f.nI, um = f.nN;
@@ -366,14 +352,15 @@ __device__ __forceinline__ FluxQ<V> face_q_split(const FaceQ<V>& f, V D, V g, V 
         const V ad = dv(one, sub(ap, am));
         const V qm = mul(Hm, um), qp = mul(Hp, up), apm = mul(ap, am);
         const V pm = mul(mul(ga, hm), mad(two, D, hm)), pp = mul(mul(ga, hp), mad(two, D, hp));
-        const V fhl = mul(mad(apm, sub(hp, hm), sub(mul(ap, qm), mul(am, qp))), ad);
-        const V ful = mul(mad(apm, sub(qp, qm), sub(mul(ap, mad(qm, um, pm)), mul(am, mad(qp, up, pp)))), ad);
+        const V nam = mul(mone, am);
+        const V fhl = mul(mad(apm, sub(hp, hm), mad(ap, qm, mul(nam, qp))), ad);
+        const V ful = mul(mad(apm, sub(qp, qm), mad(ap, mad(qm, um, pm), mul(nam, mad(qp, up, pp)))), ad);
         fh = sel(live, fhl, zero);
         fu = sel(live, ful, shift);
         a = sel(live, a, zero);
         ft = mul(sel(gt(fh, zero), f.tN, f.tI), fh);
-        sl = mul(ga, mad(sub(hp, f.hI), add(Hp, Hl), mul(add(Hl, Hi), sub(f.zri, f.eI))));
-        sr = mul(ga, mad(sub(hm, f.hN), add(Hm, Hr), mul(add(Hr, Hn), sub(f.zrn, f.eN))));
+        fq = mad(nga, mad(sub(hp, f.hI), add(Hp, Hl), mul(add(Hl, Hi), sub(f.zri, f.eI))), fu);
+        s = mad(nga, mad(sub(hm, f.hN), add(Hm, Hr), mul(add(Hr, Hn), sub(f.zrn, f.eN))), fu);
     } else {
         const V zA = vmax(sub(f.eI, f.hI), sub(f.eN, f.hN));
         const V zCN = vmin(zA, add(vmin(f.eN, f.eI), D));
@@ -393,19 +380,19 @@ __device__ __forceinline__ FluxQ<V> face_q_split(const FaceQ<V>& f, V D, V g, V 
         const V SLSR = mul(SL, SR);
         const V nSL = mul(mone, SL);
         const V fhM = mul(mad(SLSR, sub(hCNr, hCNl), mad(nSL, fhp, mul(SR, fhm))), rs);
-        const V fqM = mul(mad(SLSR, sub(fhp, fhm), mad(nSL, fup, mul(SR, fum))), rs);
+        const V fqM = mul(mad(SLSR, sub_apart(mul(hp, up), mul(hm, um)), mad(nSL, fup, mul(SR, fum))), rs);
         const auto caseL = le(zero, SL);
         const auto caseR = ge(zero, SR);
         fh = sel(caseL, fhm, sel(caseR, fhp, fhM));
         fu = sel(caseL, fum, sel(caseR, fup, fqM));
         a = vmax(vabs(SL), vabs(SR));
         ft = mul(sel(gt(fh, zero), f.tN, f.tI), fh);
-        sl = mul(mul(ga, add(Hi, add(D, hCNr))), sub(f.zri, zCN));
-        sr = mul(mul(ga, add(add(D, hCNl), Hn)), sub(f.zrn, zCN));
+        fq = mad(mul(nga, add(Hi, add(D, hCNr))), sub(f.zri, zCN), fu);
+        s = mad(mul(nga, add(add(D, hCNl), Hn)), sub(f.zrn, zCN), fu);
     }
     r.Fh = sel(r.wet, fh, zero);
-    r.Fq = sel(r.wet, sub(fu, sl), shift);
-    r.S = sel(r.wet, sub(fu, sr), shift);
+    r.Fq = sel(r.wet, fq, shift);
+    r.S = sel(r.wet, s, shift);
     r.Ft = sel(r.wet, ft, zero);
     r.a = sel(r.wet && gt(a, epsi), a, zero);
     return r;
@@ -625,6 +612,19 @@ __device__ __forceinline__ void store_ring(SmemQ<T, LANES>& s, int x, int y, T h
     if (x >= -1 && x <= BW && y >= -1 && y <= BW) BGF_ROW(s.zb, pz, x, y) = z;
 }
 
+// 1 + x / y.  Fast FP32 build: the product with the reciprocal fused into the sum.
+template <class V> __device__ __forceinline__ V one_plus_quot(V x, V y)
+{
+    using T = typename LaneOf<V>::T;
+    const V one = cst<V>((T)1.0);
+#if BGF_FAST
+    if constexpr (sizeof(T) == 4) return mad(x, rcp_v(y), one);
+    else return add_apart(one, dv(x, y));
+#else
+    return add(one, dv(x, y));
+#endif
+}
+
 // The two sides of a direction reconstructed from a cell's state and limited slopes:
 // depth, surface (engine 2: bed), normal and tangential velocity.  q: the scaled depth
 // slope over the depth (engine 1, Bouchut velocity reconstruction), wet: where it applies.
@@ -636,26 +636,16 @@ __device__ __forceinline__ void both_sides(V dx, V h, V zs, V un, V ut, V gh, V 
                                            SideQ<V>& lo, SideQ<V>& hi)
 {
     using T = typename LaneOf<V>::T;
-    const V ndx = mul(cst<V>((T)-1.0), dx), one = cst<V>((T)1.0);
+    const V ndx = mul(cst<V>((T)-1.0), dx);
     lo.h = mad(ndx, gh, h);
     hi.h = mad(dx, gh, h);
     if constexpr (ENGINE == 1) {
         lo.e = mad(ndx, gz, zs);
         hi.e = mad(dx, gz, zs);
         const auto wet = gt(Hfull, epsv);
-        const V q = dv(mul(dx, gh), Hfull);
-        V cl, ch;
-#if BGF_FAST
-        if constexpr (sizeof(T) == 4) {
-            const V qw = sel(wet, q, cst<V>((T)0.0));
-            cl = mad(qw, ndx, ndx);
-            ch = mad(qw, ndx, dx);
-        } else
-#endif
-        {
-            cl = sel(wet, mul(add(one, q), ndx), ndx);
-            ch = sel(wet, mul(sub(one, q), dx), dx);
-        }
+        const V dh = mul(dx, gh);
+        const V cl = sel(wet, mul(one_plus_quot(dh, Hfull), ndx), ndx);
+        const V ch = sel(wet, mul(one_plus_quot(mul(cst<V>((T)-1.0), dh), Hfull), dx), dx);
         lo.n = mad(cl, gn, un);
         lo.t = mad(cl, gt_, ut);
         hi.n = mad(ch, gn, un);
@@ -702,7 +692,7 @@ __device__ __forceinline__ T tile_faces(SmemQ<T, LANES>& s, const StepParams<T>&
             xp[v] = s.t[v].get(o + 1, l);
             gr[v] = slope_q<V>(th, thr, hr, xm[v], c[v], xp[v], delta, rdelta);
         }
-        if constexpr (ENGINE == 1) gr[VZS] = wetslope_q<V>(dx, c[VZS], Hc, xm[VZS], xp[VZS], gr[VZS], gr[VH], bg.gx);
+        if constexpr (ENGINE == 1) gr[VZS] = wetslope_v<V>(dx, c[VZS], Hc, xm[VZS], xp[VZS], gr[VZS], gr[VH], bg.gx);
         SideQ<V> hi;
         both_sides<V, ENGINE>(dx, c[VH], c[VZS], c[VU], c[VV], gr[VH], gr[VZS], gr[VU], gr[VV], Hc, eps, X, hi);
         const int on = pnx(x, r);
@@ -720,7 +710,7 @@ __device__ __forceinline__ T tile_faces(SmemQ<T, LANES>& s, const StepParams<T>&
             gr[v] = slope_q<V>(th, thr, hr, ym[v], c[v], s.t[v].get(o + 20, l), delta, rdelta);
         }
         // (interior rows compare both reconstructions with the lower neighbour, WetsloperesetCPU)
-        if constexpr (ENGINE == 1) gr[VZS] = wetslope_q<V>(dx, c[VZS], Hc, ym[VZS], ym[VZS], gr[VZS], gr[VH], bg.gy);
+        if constexpr (ENGINE == 1) gr[VZS] = wetslope_v<V>(dx, c[VZS], Hc, ym[VZS], ym[VZS], gr[VZS], gr[VH], bg.gy);
         SideQ<V> hi;
         both_sides<V, ENGINE>(dx, c[VH], c[VZS], c[VV], c[VU], gr[VH], gr[VZS], gr[VV], gr[VU], Hc, eps, Y, hi);
         const int on = pny(x, r);
@@ -738,7 +728,7 @@ __device__ __forceinline__ T tile_faces(SmemQ<T, LANES>& s, const StepParams<T>&
     }
     // ---- the inward sides of the 64 ring cells: two threads a cell (side tid / 32), one for
     // depth and surface, one for the velocities; slopes towards the block (the two orders of a
-    // stencil give opposite signs, exactly). 
+    // stencil give opposite signs, exactly).
     if constexpr (RingPass<T, LANES>::spread) {
         const int side = at.tid >> 5, t = (at.tid >> 1) & 15, part = at.tid & 1;
         const int hx = side == 0 ? -1 : side == 1 ? BW : t, hy = side < 2 ? t : side == 2 ? -1 : BW;
@@ -755,14 +745,9 @@ __device__ __forceinline__ T tile_faces(SmemQ<T, LANES>& s, const StepParams<T>&
             const T Hr = SPLIT ? D + n0 : n0;
             T c1 = hd_s;
             if (part == 0) {
-                g1 = wetslope_q<T>(hd_s, n1, Hr, f1, i1, g1, g0, bg.ring);
+                g1 = wetslope_v<T>(hd_s, n1, Hr, f1, i1, g1, g0, bg.ring);
                 // the velocities' factor (both_sides)
-                const T q = dv(mul(hd_s, g0), Hr);
-#if BGF_FAST
-                if constexpr (sizeof(T) == 4) c1 = mad(sel(gt(Hr, p.epsface), q, (T)0.0), -hd_s, hd_s);
-                else
-#endif
-                    c1 = sel(gt(Hr, p.epsface), mul(sub((T)1.0, q), hd_s), hd_s);
+                c1 = sel(gt(Hr, p.epsface), mul(one_plus_quot(-mul(hd_s, g0), Hr), hd_s), hd_s);
             }
             c1 = __shfl_sync(0xffffffffu, c1, lane & ~1);
             if (part == 0) c1 = hd_s;
@@ -802,7 +787,7 @@ __device__ __forceinline__ T tile_faces(SmemQ<T, LANES>& s, const StepParams<T>&
             if (j == 1) { zm = m0; zp = p0; }
         }
         const T Hr = SPLIT ? D + q0[0] : q0[0];
-        if constexpr (ENGINE == 1) gr[1] = wetslope_q<T>(hd_s, q0[1], Hr, zm, zp, gr[1], gr[0], bg.ring);
+        if constexpr (ENGINE == 1) gr[1] = wetslope_v<T>(hd_s, q0[1], Hr, zm, zp, gr[1], gr[0], bg.ring);
         SideQ<T> in, outw;
         // (both_sides with the signed half spacing: its high side is the inward one)
         both_sides<T, ENGINE>(sg, q0[0], q0[1], q0[2], q0[3], gr[0], gr[1], gr[2], gr[3], Hr, p.epsface, outw, in);
@@ -1057,10 +1042,10 @@ template <class T> __device__ __forceinline__ T finite_speed(V2<T> h, V2<T> u, V
 {
 #if BGF_FAST
     if constexpr (sizeof(T) == 4) {
-        // one test for both cells: the sum is finite exactly when all six values are (a NaN or
-        // an infinity carries through it; finite states are far below the float range)
+        // one test per cell: the sum is finite exactly when h, u and v are (a NaN or an
+        // infinity carries through it; finite states are far below the float range)
         const V2<T> q = add(add(h, u), v);
-        return isfinite(q.a + q.b) ? a : (T)INFINITY;
+        return isfinite(q.a) && isfinite(q.b) ? a : (T)INFINITY;
     }
 #endif
     return finite_speed<T>(h.a, u.a, v.a, finite_speed<T>(h.b, u.b, v.b, a));
