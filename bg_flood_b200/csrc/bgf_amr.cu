@@ -613,7 +613,7 @@ __global__ void __launch_bounds__(Quad<T, amr_lanes<T>()>::NT, AmrOcc<T>::step)
     const V hold = own_of<V>(m.h[ts.cur], g, 128, at.l), uold = own_of<V>(m.u[ts.cur], g, 128, at.l),
             vold = own_of<V>(m.v[ts.cur], g, 128, at.l);
     const int nxt = ts.cur ^ 1;
-    full_step<T, false, LANES>(m, p, ib, at, g, nxt, dt, delta, (T)0, s.rainv, ts.totaltime, hold, uold, vold, dh, dhu, dhv);
+    full_step<T, false, LANES, true>(m, p, ib, at, g, nxt, dt, delta, (T)0, s.rainv, ts.totaltime, hold, uold, vold, dh, dhu, dhv);
     if (lead && tid == 0) m.time[2 * sc + (parity ^ 1)] = next_time_state<T>(ts, p, dtd, nxt, m.dtmin + 2 * sc, parity);
 }
 

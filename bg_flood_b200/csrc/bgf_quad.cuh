@@ -1082,21 +1082,44 @@ __device__ __forceinline__ T add_rivers_q(const DevModel<T>& m, const StepParams
                          p.xo_d + m.bxo[ib], p.yo_d + m.byo[ib], x, y, dh, time);
 }
 
+// The full step and the friction of one cell as the multi-level chain's other kernels
+// (StageState) make them: plain divisions and cube root.
+template <class T>
+__device__ __forceinline__ void plain_step(const StepParams<T>& p, T dt, T cf, T hold, T uold, T vold, T dh, T dhu, T dhv,
+                                           T& ho, T& uo, T& vo)
+{
+    advance<T>(dt, p.eps, p.eps_d, p.forcemass != 0, hold, uold, vold, dh, dhu, dhv, ho, uo, vo);
+    bottom_friction<T>(p.frictionmodel, p.g, p.eps, dt, cf, ho, uo, vo);
+}
+
 // Full step of the own cells from state n (AdvkernelCPU with evolv), then friction on the
-// result and rain; the next state goes to buffer nxt.
-template <class T, bool SPLIT, int LANES, class V>
+// result and rain; the next state goes to buffer nxt.  PLAIN: with the compiler's divisions
+// (fast build: full range) instead of products with the reciprocal, cell by cell.
+template <class T, bool SPLIT, int LANES, bool PLAIN = false, class V>
 __device__ __forceinline__ void full_step(const DevModel<T>& m, const StepParams<T>& p, int ib, const Place<T, LANES>& at,
                                           size_t g, int nxt, T dt, T delta, T D, T rainv, double time, V hold, V uold,
                                           V vold, V dh, V dhu, V dhv)
 {
     const bool fm = p.forcemass != 0;
     const V Dv = cst<V>(D);
-    V ho, uo, vo;
-    if constexpr (SPLIT) advance_split_v<V>(dt, p.eps, fm, Dv, hold, uold, vold, dh, dhu, dhv, ho, uo, vo);
-    else advance_v<V>(dt, p.eps, p.eps_d, fm, hold, uold, vold, dh, dhu, dhv, ho, uo, vo);
     const V cfv = p.has_cf ? own_of<V>(m.cf, g, 128, at.l) : cst<V>(p.cf);
-    // (split precision: friction on the full depth; the deviation is not changed by it)
-    friction_v<V>(p.frictionmodel, p.g, p.eps, dt, cfv, SPLIT ? add(Dv, ho) : ho, uo, vo);
+    V ho, uo, vo;
+    if constexpr (PLAIN && LANES == 1) {
+        plain_step<T>(p, dt, cfv, hold, uold, vold, dh, dhu, dhv, ho, uo, vo);
+    } else if constexpr (PLAIN) {
+        plain_step<T>(p, dt, cfv.a, hold.a, uold.a, vold.a, dh.a, dhu.a, dhv.a, ho.a, uo.a, vo.a);
+        plain_step<T>(p, dt, cfv.b, hold.b, uold.b, vold.b, dh.b, dhu.b, dhv.b, ho.b, uo.b, vo.b);
+    } else {
+        if constexpr (SPLIT) advance_split_v<V>(dt, p.eps, fm, Dv, hold, uold, vold, dh, dhu, dhv, ho, uo, vo);
+        else advance_v<V>(dt, p.eps, p.eps_d, fm, hold, uold, vold, dh, dhu, dhv, ho, uo, vo);
+        // (split precision: friction on the full depth; the deviation is not changed by it)
+        friction_v<V>(p.frictionmodel, p.g, p.eps, dt, cfv, SPLIT ? add(Dv, ho) : ho, uo, vo);
+    }
+    auto quot = [](V x, V y) {
+        if constexpr (!PLAIN) return dv(x, y);
+        else if constexpr (LANES == 1) return x / y;
+        else return V{x.a / y.a, x.b / y.b};
+    };
     if (p.has_rain) {
         // AddrainforcingImplicitCPU (src/Updateforcing.cu:530-580): the rain rate at
         // the start of the step, uniform or gridded
@@ -1109,13 +1132,13 @@ __device__ __forceinline__ void full_step(const DevModel<T>& m, const StepParams
             };
             if constexpr (LANES == 1) Rainhh = rate(at.r + 8 * at.l);
             else Rainhh = V{rate(at.r), rate(at.r + 8)};
-            const V rr = dv(dv(Rainhh, cst<V>((T)1000.0)), cst<V>((T)3600.0));
+            const V rr = quot(quot(Rainhh, cst<V>((T)1000.0)), cst<V>((T)3600.0));
             Rainhh = mul(vmax(mul(rr, cst<V>(dt)), cst<V>((T)0.0)), mask);
         } else {
             Rainhh = mul(cst<V>(rainv), mask);  // (the block's uniform depth, above)
         }
         const V hi = SPLIT ? add(Dv, ho) : ho;
-        const V qvol = dv(hi, add(hi, Rainhh));
+        const V qvol = quot(hi, add(hi, Rainhh));
         ho = add(ho, Rainhh);
         typename LaneOf<V>::Mask wet;
         if constexpr (LANES == 1) wet = (double)hi > p.eps_d;

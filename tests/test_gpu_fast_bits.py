@@ -6,14 +6,17 @@ rounded products and sums, one reciprocal per star region, upwind fluxes taken a
 
 Signed zeros count as equal; everything else must be the same bits."""
 import hashlib
+import os
 
 import numpy as np
 import pytest
 
 import cases
-from runners import interior, make_gpu
+from runners import interior, make_gpu, make_gpu_amr
 
 pytestmark = pytest.mark.gpu
+
+GOLDEN = os.path.join(os.path.dirname(__file__), "golden")
 
 
 def _set(case, **kw):
@@ -43,6 +46,15 @@ def _island(n, engine, **kw):
     return _set(c, **kw)
 
 
+def _amr(name, mk, rain=None, **kw):
+    g = np.load(os.path.join(GOLDEN, f"{name}.npz"))
+    case = _set(mk(), **kw)
+    f, loop = make_gpu_amr(case, (g["level"], g["nbr"], g["xo"], g["yo"]))
+    if rain:
+        f.set_rain(*rain)
+    return f, loop
+
+
 def _reg(case):
     f, _, loop = make_gpu(case)
     return f, loop
@@ -70,11 +82,18 @@ RUNS = {
     "island_e2": (lambda: _reg(_island(96, 2)), 80),
     "rain_e1": (lambda: _reg(_set(cases.rain_on_terrain(64, 1))), 60),
     "dam_e1_sources": (lambda: _sources(_reg(_set(cases.dam_break(64, 1), cf=0.03, frictionmodel=-1)), 32.0), 60),
+    "amr_dam_e1_sources": (lambda: _sources(_amr("amrdam64_e1_l2", lambda: cases.amr_dambreak(64, 1, 2)), 32.0), 60),
     "tsunami_split": (lambda: _reg(_set(cases.ensemble_member(3, 2024, 64, 512), splitprecision=1)), 40),
     "chute_e1_split": (lambda: _reg(_chute(1, splitprecision=1)), 80),
     "chute_e2_split": (lambda: _reg(_chute(2, splitprecision=1)), 60),
     "island_e1_split": (lambda: _reg(_island(64, 1, splitprecision=1)), 40),
     "rain_e1_split": (lambda: _reg(_set(cases.rain_on_terrain(64, 1), splitprecision=1)), 40),
+    "amr_dam_e1_l3": (lambda: _amr("amrdam64_e1_l3", lambda: cases.amr_dambreak(64, 1, 3)), 60),
+    "amr_dam_e1_l2_rain": (lambda: _amr("amrdam64_e1_l2", lambda: cases.amr_dambreak(64, 1, 2),
+                                        ([0.0, 1e9], [80.0, 80.0]), cf=0.03, frictionmodel=-1, lat=45.0), 60),
+    "amr_dam_e2_l2_smart": (lambda: _amr("amrdam64_e2_l2", lambda: cases.amr_dambreak(64, 2, 2), cf=0.01,
+                                         frictionmodel=1, lat=45.0), 60),
+    "amr_hump_e2_l2": (lambda: _amr("amrhump64_e2_l2", lambda: cases.amr_hump(64, 2, 2, 0.3)), 40),
 }
 
 
@@ -96,6 +115,7 @@ def digest(name):
 
 
 DIGESTS = {
+    "amr_dam_e1_sources": "5a9ce8073db50000",
     "dam_e1_sources": "5d9c0eaf2f43f3c8",
     "gauss_e1_absorbing": "94cfea69c87b4ad6",
     "gauss_e2_absorbing": "886228ac31590571",
@@ -113,6 +133,10 @@ DIGESTS = {
     "chute_e2_split": "69a7c53aa0291e2d",
     "island_e1_split": "68af487876c244fd",
     "rain_e1_split": "69fecb6642e23d1c",
+    "amr_dam_e1_l3": "eb4b83c392ab80fd",
+    "amr_dam_e1_l2_rain": "75c26a14ed11b5ac",
+    "amr_dam_e2_l2_smart": "f7295b3cf42f5a0c",
+    "amr_hump_e2_l2": "d4d35620842fa2a9",
 }
 
 
