@@ -1797,6 +1797,27 @@ static int finish_step(bgf_handle* h, bgf_loop* loop, int err, const TimeState& 
     return BGF_OK;
 }
 
+// Stream capture of a graph.  The enqueue functions leave the errors of launches and of the
+// multi-level fork to cudaGetLastError: end_capture looks, and gives up a graph from which a
+// kernel may be missing.
+static int begin_capture(cudaStream_t st)
+{
+    cudaGetLastError();  // (one left by an earlier call is not the capture's)
+    BGF_CUDA(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal));
+    return BGF_OK;
+}
+static int end_capture(cudaStream_t st, cudaGraph_t* g)
+{
+    const cudaError_t el = cudaGetLastError();
+    cudaError_t e = cudaStreamEndCapture(st, g);
+    if (e == cudaSuccess && el != cudaSuccess) cudaGraphDestroy(*g);
+    if (el != cudaSuccess) e = el;
+    if (e == cudaSuccess) return BGF_OK;
+    cudaGetLastError();
+    g_last_error = std::string("graph capture: ") + cudaGetErrorString(e);
+    return BGF_ECUDA;
+}
+
 // One flow step for parity p as a graph: one copy of the control block's time and
 // dt slots in (slot p carries the step's loop state; the other slots are overwritten
 // by the step itself), the step's kernels, and one copy out from time slot p ^ 1 to
@@ -1804,18 +1825,15 @@ static int finish_step(bgf_handle* h, bgf_loop* loop, int err, const TimeState& 
 static int build_step_graph(bgf_handle* h, int p)
 {
     cudaGraph_t g;
-    BGF_CUDA(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
+    int rc = begin_capture(h->stream);
+    if (rc) return rc;
     cudaMemcpyAsync(h->d_ctl, h->h_ctl, offsetof(StepCtl, err), cudaMemcpyHostToDevice, h->stream);
     h->step_graph_launches[p] = h->dbl ? enqueue_step<double>(h, p) : enqueue_step<float>(h, p);
     const size_t off = offsetof(StepCtl, t) + (size_t)(p ^ 1) * sizeof(TimeState);
     cudaMemcpyAsync((char*)h->h_ctl + off, (const char*)h->d_ctl + off, offsetof(StepCtl, err) + sizeof(int) - off,
                     cudaMemcpyDeviceToHost, h->stream);
-    cudaError_t e = cudaStreamEndCapture(h->stream, &g);
-    if (e != cudaSuccess) {
-        g_last_error = std::string("graph capture: ") + cudaGetErrorString(e);
-        return BGF_ECUDA;
-    }
-    e = cudaGraphInstantiate(&h->step_graph[p], g, 0);
+    if ((rc = end_capture(h->stream, &g))) return rc;
+    cudaError_t e = cudaGraphInstantiate(&h->step_graph[p], g, 0);
     cudaGraphDestroy(g);
     if (e != cudaSuccess) {
         h->step_graph[p] = nullptr;
@@ -1891,17 +1909,14 @@ constexpr int kLongRun = 16;
 static int build_run_graph(bgf_handle* h, int p0, int steps, cudaGraphExec_t* out)
 {
     cudaGraph_t g;
-    BGF_CUDA(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
+    int rc = begin_capture(h->stream);
+    if (rc) return rc;
     int n = 0;
     for (int k = 0; k < steps; k++)
         n += h->dbl ? enqueue_step<double>(h, p0 ^ (k & 1)) : enqueue_step<float>(h, p0 ^ (k & 1));
     h->steps_launches = n / steps;
-    cudaError_t e = cudaStreamEndCapture(h->stream, &g);
-    if (e != cudaSuccess) {
-        g_last_error = std::string("graph capture: ") + cudaGetErrorString(e);
-        return BGF_ECUDA;
-    }
-    e = cudaGraphInstantiate(out, g, 0);
+    if ((rc = end_capture(h->stream, &g))) return rc;
+    cudaError_t e = cudaGraphInstantiate(out, g, 0);
     cudaGraphDestroy(g);
     if (e != cudaSuccess) {
         *out = nullptr;

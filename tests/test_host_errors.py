@@ -1,0 +1,101 @@
+"""The library's host code when a call of the CUDA runtime fails, on the CPU: its own objects
+are linked with a stand-in for the runtime (fake_cudart.cpp), whose calls a test lets fail."""
+import ctypes
+import os
+import subprocess
+
+import numpy as np
+import pytest
+
+import bg_flood_b200._native as native
+import bg_flood_b200.build as build
+import cases
+from bg_flood_b200.flow import BGFError, Loop
+from runners import make_gpu, make_gpu_amr
+
+HERE = os.path.dirname(os.path.abspath(__file__))
+EINVAL, ECUDA = 1, 2
+
+
+@pytest.fixture(scope="module")
+def fake_lib(tmp_path_factory):
+    objs = [os.path.join(build.LIBDIR, o) for _, o, _ in build.SOURCES]
+    if not all(os.path.exists(o) for o in objs):
+        build.build(force=True)
+    out = str(tmp_path_factory.mktemp("fake") / "libfake.so")
+    cuda = os.path.join(os.path.dirname(os.path.dirname(build.nvcc())), "include")
+    subprocess.run(["g++", "-O1", "-std=c++17", "-fPIC", "-shared", "-I", cuda, os.path.join(HERE, "fake_cudart.cpp"), *objs,
+                    "-Wl,-Bsymbolic", "-lpthread", "-o", out], check=True)
+    l = ctypes.CDLL(out)
+    for name, (res, args) in native.SIGNATURES.items():
+        getattr(l, name).restype, getattr(l, name).argtypes = res, args
+    l.fake_fail.argtypes = [ctypes.c_char_p, ctypes.c_int]
+    l.fake_calls.argtypes = [ctypes.c_char_p]
+    return l
+
+
+@pytest.fixture
+def fake(fake_lib, monkeypatch):
+    monkeypatch.setattr(native, "_lib", fake_lib)
+    failing = set()
+
+    def fail(name, nth=1):
+        failing.add(name)
+        fake_lib.fake_fail(name.encode(), nth)
+
+    fail.calls = lambda name: fake_lib.fake_calls(name.encode())
+    fail.graphs = fake_lib.fake_live_graphs
+    yield fail
+    for name in failing:
+        fake_lib.fake_fail(name.encode(), 0)
+
+
+def _single():
+    f, _, loop = make_gpu(cases.hump_walls(64, 1))
+    loop.nextoutputtime = 1e30
+    loop.dtmax = 1.0
+    return f, loop
+
+
+def _amr(name="amrdam64_e1_l2"):
+    g = np.load(os.path.join(HERE, "golden", f"{name}.npz"))
+    return make_gpu_amr(cases.amr_dambreak(64, 1, 2), (g["level"], g["nbr"], g["xo"], g["yo"]))
+
+
+def _raises(status, call):
+    with pytest.raises(BGFError) as e:
+        call()
+    assert e.value.status == status
+
+
+@pytest.mark.parametrize("call", ["step", "run"])
+@pytest.mark.parametrize("mk,name", [(_single, "cudaLaunchKernelExC"), (_amr, "cudaLaunchKernelExC"),
+                                     (_amr, "cudaEventRecord"), (_amr, "cudaStreamWaitEvent")],
+                         ids=["launch", "amr_launch", "fork_record", "fork_wait"])
+def test_a_graph_without_one_of_its_launches_is_not_kept(fake, mk, name, call):
+    """A launch, or the fork of the multi-level branches, that fails while a graph is captured:
+    the call reports it and the next one builds the graph anew."""
+    f, loop = mk()
+    go = (lambda: f.flow_step(loop)) if call == "step" else (lambda: f.run(loop, 1e30, maxsteps=2))
+    fake("cudaGraphLaunch", 0)
+    fake(name)
+    _raises(ECUDA, go)
+    assert fake.calls("cudaGraphLaunch") == 0 and fake.graphs() == 0
+    fake(name, 0)
+    fake("cudaStreamBeginCapture", 0)
+    go()
+    assert fake.calls("cudaStreamBeginCapture") == 1 and fake.calls("cudaGraphLaunch") == 1
+    f.close()
+
+
+def test_a_failed_pool_graph_is_not_kept(fake):
+    from bg_flood_b200.pool import ScenarioPool
+    f, loop = _single()
+    pool = ScenarioPool(cases.hump_walls(64, 1).param, 64, 2)
+    pool.admit(f, loop, 1e30, maxsteps=4)
+    fake("cudaLaunchKernelExC")
+    _raises(ECUDA, lambda: pool.run(4))
+    fake("cudaLaunchKernelExC", 0)
+    pool.run(4)
+    assert fake.graphs() == 0
+    pool.close()
