@@ -972,14 +972,15 @@ static int rebuild_segments(bgf_handle* h);
 static int alloc_amr(bgf_handle* h)
 {
     if (h->d_rank) return BGF_OK;
+    // (each by itself: an attempt may have failed between them)
     if (!h->stream2) {
         // (at the priority of the main stream: both branches share the SMs)
         int prio = 0;
         if (cudaStreamGetPriority(h->stream, &prio) != cudaSuccess) prio = 0;
         BGF_CUDA(cudaStreamCreateWithPriority(&h->stream2, cudaStreamNonBlocking, prio));
-        BGF_CUDA(cudaEventCreateWithFlags(&h->ev_fork, cudaEventDisableTiming));
-        BGF_CUDA(cudaEventCreateWithFlags(&h->ev_join, cudaEventDisableTiming));
     }
+    if (!h->ev_fork) BGF_CUDA(cudaEventCreateWithFlags(&h->ev_fork, cudaEventDisableTiming));
+    if (!h->ev_join) BGF_CUDA(cudaEventCreateWithFlags(&h->ev_join, cudaEventDisableTiming));
     const size_t nb = (size_t)h->nblkmem, es = h->esz;
     bool ok = true;
     for (auto& st : h->d_W)

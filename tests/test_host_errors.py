@@ -99,3 +99,28 @@ def test_a_failed_pool_graph_is_not_kept(fake):
     pool.run(4)
     assert fake.graphs() == 0
     pool.close()
+
+
+@pytest.mark.parametrize("name,nth", [("cudaStreamCreateWithPriority", 1), ("cudaEventCreateWithFlags", 1),
+                                      ("cudaEventCreateWithFlags", 2)])
+def test_the_second_branch_is_complete_or_absent(fake, name, nth):
+    """The stream and the two events of the multi-level fork: after one could not be made, the
+    next attempt makes what is missing."""
+    f, loop = _amr()  # (its tables once more, on a new handle whose first attempt fails)
+    blocks = f.get_blocks()
+    f.close()
+    from bg_flood_b200.flow import FlowB200
+    case = cases.amr_dambreak(64, 1, 2)
+    g = np.load(os.path.join(HERE, "golden", "amrdam64_e1_l2.npz"))
+    n = len(g["level"])
+    f = FlowB200(case.param, n)
+    set_blocks = lambda: f.set_blocks(np.arange(n, dtype=np.int32), g["level"], g["nbr"], g["xo"], g["yo"])
+    fake(name, nth)
+    _raises(ECUDA, set_blocks)
+    fake(name, 0)
+    set_blocks()
+    zero = np.zeros((n, 18, 18))
+    f.set_bed(zero)
+    f.set_state(zero + 1, zero, zero)
+    f.flow_step(loop)
+    f.close()
