@@ -1949,6 +1949,24 @@ static int launch_run(bgf_handle* h, int p0, int nlong, int npair)
     return BGF_OK;
 }
 
+// Launches a batch's graphs and reads the time state they end in, also when a launch failed
+// and only some of them ran.
+static int run_batch(bgf_handle* h, int p0, int nlong, int npair, double* gpu_ms, int64_t* launched, TimeState* ts)
+{
+    BGF_CUDA(cudaEventRecord(h->ev0, h->stream));
+    const int rc = launch_run(h, p0, nlong, npair);
+    BGF_CUDA(cudaEventRecord(h->ev1, h->stream));
+    if (!rc) *launched += (int64_t)h->steps_launches * (nlong * kLongRun + 2 * npair);
+    // after whole graphs the latest time state is in slot p0
+    BGF_CUDA(cudaMemcpyAsync(&h->h_time[1], h->d_time + p0, sizeof(TimeState), cudaMemcpyDeviceToHost, h->stream));
+    BGF_CUDA(cudaStreamSynchronize(h->stream));
+    float ms = 0.f;
+    cudaEventElapsedTime(&ms, h->ev0, h->ev1);
+    *gpu_ms += ms;
+    *ts = h->h_time[1];
+    return rc;
+}
+
 int bgf_run(bgf_handle* h, bgf_loop* loop, double endtime, double outputtimestep, int maxsteps, int* nsteps)
 {
     int rc = check_ready(h);
@@ -1967,28 +1985,18 @@ int bgf_run(bgf_handle* h, bgf_loop* loop, double endtime, double outputtimestep
         long long left = (long long)maxsteps - ts.nstep;
         long long want = (long long)std::min<double>(remaining * 1.02 + 2.0, (double)left);
         int nlong = 0, npair = 0;
-        if ((rc = prepare_run(h, p0, (int)std::max<long long>(1, std::min<long long>(want, 1024)), &nlong, &npair))) return rc;
-        BGF_CUDA(cudaEventRecord(h->ev0, h->stream));
-        if ((rc = launch_run(h, p0, nlong, npair))) return rc;
-        BGF_CUDA(cudaEventRecord(h->ev1, h->stream));
-        launched += (int64_t)h->steps_launches * (nlong * kLongRun + 2 * npair);
-        // after whole graphs the latest time state is in slot p0
-        BGF_CUDA(cudaMemcpyAsync(&h->h_time[1], h->d_time + p0, sizeof(TimeState), cudaMemcpyDeviceToHost, h->stream));
-        BGF_CUDA(cudaStreamSynchronize(h->stream));
-        float ms = 0.f;
-        cudaEventElapsedTime(&ms, h->ev0, h->ev1);
-        gpu_ms += ms;
-        ts = h->h_time[1];
+        if ((rc = prepare_run(h, p0, (int)std::max<long long>(1, std::min<long long>(want, 1024)), &nlong, &npair))) break;
+        if ((rc = run_batch(h, p0, nlong, npair, &gpu_ms, &launched, &ts))) break;
         // at most 1024 steps per batch: the 4096-sample gauge ring cannot overflow
-        if ((rc = gauge_drain_handle(h))) return rc;
+        if ((rc = gauge_drain_handle(h))) break;
         if (ts.dt > 0) dtguess = ts.dt;
         if (ts.done || ts.totaltime >= endtime || ts.nstep >= maxsteps) break;
     }
     h->launches += launched;
     h->last_run_ms = gpu_ms;
     h->last_run_launches = launched;
-    rc = check_err_word(h);
-    if (rc) return rc;
+    if (!rc && (rc = check_err_word(h))) return rc;
+    // (also where a later batch failed: the steps before it are in the device's state)
     loop->totaltime = ts.totaltime;
     loop->dt = ts.dt;
     loop->dtmax = ts.dtmax;
@@ -1996,6 +2004,7 @@ int bgf_run(bgf_handle* h, bgf_loop* loop, double endtime, double outputtimestep
     h->cur = ts.cur;
     // parity stays p0: every graph replay advances it by two
     if (nsteps) *nsteps = (int)ts.nstep;
+    if (rc) return rc;
     if (ts.status == BGF_EDT_UNDERFLOW || ts.status == BGF_ENAN) return ts.status;
     return BGF_OK;
 }

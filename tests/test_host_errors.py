@@ -124,3 +124,18 @@ def test_the_second_branch_is_complete_or_absent(fake, name, nth):
     f.set_state(zero + 1, zero, zero)
     f.flow_step(loop)
     f.close()
+
+
+@pytest.mark.parametrize("name,nth", [("cudaGraphInstantiate", 2), ("cudaStreamBeginCapture", 2), ("cudaGraphLaunch", 66)])
+def test_a_run_that_fails_in_a_later_batch_keeps_its_progress(fake, name, nth):
+    """1024 steps in graphs of 16, then 4 more in graphs of two, whose graph cannot be built or
+    launched: the loop is where the device is, and another run goes on from there."""
+    f, loop = _single()
+    fake(name, nth)
+    _raises(ECUDA, lambda: f.run(loop, 1e30, maxsteps=1028))
+    done = loop.totaltime
+    assert done == (1026.0 if name == "cudaGraphLaunch" else 1024.0)  # (a step is a second here)
+    fake(name, 0)
+    n = f.run(loop, 1e30, maxsteps=1028 - int(done))
+    assert n == 1028 - int(done) and loop.totaltime == 1028.0
+    f.close()
