@@ -117,6 +117,7 @@ struct bgf_handle {
     // graphs of two and of kLongRun consecutive steps from parity p (built when first used)
     cudaGraphExec_t graph[2] = {nullptr, nullptr};
     cudaGraphExec_t graph_long[2] = {nullptr, nullptr};
+    int64_t graph_steps = 0;  // steps asked of runs since the graphs were last dropped
     // graph of one bgf_flow_step per parity: time-slot upload, the step, result download
     cudaGraphExec_t step_graph[2] = {nullptr, nullptr};
     int step_graph_launches[2] = {0, 0};
@@ -344,6 +345,7 @@ static unsigned long long dt_init_bits(int dbl)
 
 static void free_graphs(bgf_handle* h)
 {
+    h->graph_steps = 0;
     for (int k = 0; k < 2; k++) {
         if (h->graph[k]) {
             cudaGraphExecDestroy(h->graph[k]);
@@ -1906,6 +1908,10 @@ int bgf_flow_step(bgf_handle* h, bgf_loop* loop)
 // (programmatic dependent launch); between two graphs they do not.  A run replays long
 // graphs for as many steps as fit and graphs of two for the rest.
 constexpr int kLongRun = 16;
+// The long graph pays from here on: it takes some 200 us to build and saves about 3.5 us a step,
+// so that the first run of a fresh handle took longer with it up to 40 steps (128x128 cells, 20
+// steps: 545 us, 520 with graphs of two for both parities).
+constexpr int kLongAfter = 64;
 
 static int build_run_graph(bgf_handle* h, int p0, int steps, cudaGraphExec_t* out)
 {
@@ -1934,8 +1940,10 @@ static int prepare_run(bgf_handle* h, int p0, int steps, int* nlong, int* npair)
     const int pairs = std::max(1, (steps + 1) / 2);
     // (a multi-level step is up to 18 launches, most of them not chained: a long graph would
     // cost more to build after each refinement pass than it saves)
-    *nlong = h->amr ? 0 : pairs / (kLongRun / 2);
-    *npair = h->amr ? pairs : pairs % (kLongRun / 2);
+    h->graph_steps += 2 * pairs;
+    const bool lg = !h->amr && (h->graph_long[p0] || h->graph_steps >= kLongAfter);
+    *nlong = lg ? pairs / (kLongRun / 2) : 0;
+    *npair = lg ? pairs % (kLongRun / 2) : pairs;
     int rc = BGF_OK;
     if (*nlong && !h->graph_long[p0] && (rc = build_run_graph(h, p0, kLongRun, &h->graph_long[p0]))) return rc;
     if (*npair && !h->graph[p0]) rc = build_run_graph(h, p0, 2, &h->graph[p0]);

@@ -139,3 +139,27 @@ def test_a_run_that_fails_in_a_later_batch_keeps_its_progress(fake, name, nth):
     n = f.run(loop, 1e30, maxsteps=1028 - int(done))
     assert n == 1028 - int(done) and loop.totaltime == 1028.0
     f.close()
+
+
+def test_graphs_a_run_builds(fake):
+    """The graph of 16 steps is built once the runs of a handle would replay it often enough,
+    not for a short first run; setting something that drops the graphs starts anew."""
+    f, loop = _single()
+
+    def built(steps):
+        fake("cudaGraphInstantiate", 0)
+        fake("cudaGraphLaunch", 0)
+        assert f.run(loop, 1e30, maxsteps=steps) == steps
+        return fake.calls("cudaGraphInstantiate"), fake.calls("cudaGraphLaunch")
+
+    assert built(20) == (1, 10)
+    assert built(20) == (0, 10)
+    assert built(20) == (0, 10)
+    assert built(20) == (1, 3)      # (80 steps in all: from here on one of 16 and two of two)
+    assert built(33) == (0, 3)
+    f.set_rain([0.0, 1e9], [1.0, 1.0])
+    assert built(20) == (1, 10)
+    f.close()
+    f, loop = _single()
+    assert built(100) == (2, 8)
+    f.close()
