@@ -251,11 +251,20 @@ def cpu_baseline_entry(r: dict) -> dict:
             "host": hc, "taskset_cores": sorted(os.sched_getaffinity(0)) if hasattr(os, "sched_getaffinity") else None}
 
 
+def reference_missing() -> str | None:
+    """Why the reference's own code cannot run here (None: it can)."""
+    from oracle.pyoracle import ref_available
+    return None if ref_available() else "oracle/_ref/libbgf_ref.so is not built (the reference's sources are absent)"
+
+
 def reference_gpu_baseline(n: int, engine: int, steps: int) -> dict:
     """The reference's own FlowGPU (its CUDA sources compiled for sm_100a by
     oracle/ref/Makefile) on the same workload and GPU, through the oracle harness:
     wall clock of `steps` steps after 3 untimed ones (each reference step reads its dt
     back to the host, so the clock covers its work), and its distance from FlowCPU."""
+    why = reference_missing()
+    if why:
+        return {"unavailable": why}
     import torch
     from runners import interior, make_oracle, make_reference
     case = workload_case(n, engine, 0, 0)
@@ -282,6 +291,9 @@ def accuracy_full_run(n: int, engine: int, dev: int, fastmath: int, endtime: flo
     headline build against the reference's own FP64 FlowGPU (its CUDA sources built
     for sm_100a) over the same simulated time, both on this GPU: max |eta|, |hu|,
     |hv| over all cells at the end, and the step counts."""
+    why = reference_missing()
+    if why:
+        return {"unavailable": why}
     import torch
     from runners import interior, make_gpu, make_reference
     case = workload_case(n, engine, dev, fastmath)
@@ -709,6 +721,10 @@ def _serving_at_rate(nreq: int, seed: int, rate: float, dev: int, fastmath: int,
 
 def run_reference_arm(args, rank, world):
     if rank != 0:
+        return
+    why = reference_missing()
+    if why:
+        print(json.dumps({"impl": "reference", "unavailable": why}), flush=True)
         return
     steps = max(1, args.steps if args.steps <= 20 else 10)
     r = cpu_reference_sample(steps, min(args.warmup, 3), args.engine, "O2")
