@@ -1,10 +1,11 @@
-"""The thread layouts of the fused single-level kernels (bgf_set_kernel_layout: one
-cell per thread, two cells per thread, or two cells per thread in persistent CTAs
-whose producer warp stages each block's tile with bulk asynchronous copies) give
-the same results: bit for bit in the exact build, within the fast-math tolerance in
-the fast build (there the two-cell kernels use paired FP32 instructions and
-contract other products into fused multiply-adds).  All run through the C ABI on
-the same inputs, handles and pools."""
+"""The thread layouts of the fused single-level kernels (bgf_set_kernel_layout: 1 the separate
+one-cell kernels, 2 the pair kernels; 3 is another name of 2) give the same results: bit for
+bit in the exact build, within the fast-math tolerance in the fast build (there the pair
+kernels use paired FP32 instructions, fuse other products into sums and divide by reciprocals).
+All run through the C ABI on the same inputs, handles and pools.
+
+The meshes here are small; in the exact build the pair kernels then take one cell per thread.
+Their pairs are compared in test_gpu_quad.py, on meshes of 700 blocks and more."""
 import numpy as np
 import pytest
 
@@ -41,46 +42,50 @@ def _run(mk, layout, fast, nsteps, dbl=False):
     return dts, f.get_state()
 
 
-@pytest.mark.parametrize("layout", [2, 3])
 @pytest.mark.parametrize("name,mk,nsteps", CASES, ids=[c[0] for c in CASES])
-def test_layouts_bit_identical_exact(name, mk, nsteps, layout):
+def test_layouts_bit_identical_exact(name, mk, nsteps):
     d1, s1 = _run(mk, 1, 0, nsteps)
-    d2, s2 = _run(mk, layout, 0, nsteps)
+    d2, s2 = _run(mk, 2, 0, nsteps)
     assert d1 == d2
     for k, a, b in zip("zs h u v".split(), s1, s2):
         assert np.array_equal(interior(a), interior(b)), (k, float(np.abs(interior(a) - interior(b)).max()))
 
 
-@pytest.mark.parametrize("layout", [2, 3])
 @pytest.mark.parametrize("name,mk,nsteps", CASES, ids=[c[0] for c in CASES])
-def test_layouts_close_fast(name, mk, nsteps, layout):
+def test_layouts_close_fast(name, mk, nsteps):
     d1, s1 = _run(mk, 1, 1, nsteps)
-    d2, s2 = _run(mk, layout, 1, nsteps)
+    d2, s2 = _run(mk, 2, 1, nsteps)
     for a, b in zip(d1, d2):
         assert abs(a - b) <= FAST_DT_RTOL * a
     for k, a, b in zip("zs h u v".split(), s1, s2):
         assert float(np.abs(interior(a).astype(np.float64) - interior(b)).max()) <= FAST_TOL, k
 
 
-@pytest.mark.parametrize("layout", [2, 3])
-def test_layouts_bit_identical_double(layout):
+def test_layout_3_is_layout_2():
+    for fast in (0, 1):
+        d2, s2 = _run(CASES[3][1], 2, fast, 20)
+        d3, s3 = _run(CASES[3][1], 3, fast, 20)
+        assert d2 == d3 and all(np.array_equal(interior(a), interior(b)) for a, b in zip(s2, s3))
+
+
+def test_layouts_bit_identical_double():
     mk = lambda: cases.dam_break(32, 1)
     d1, s1 = _run(mk, 1, 0, 30, dbl=True)
-    d2, s2 = _run(mk, layout, 0, 30, dbl=True)
+    d2, s2 = _run(mk, 2, 0, 30, dbl=True)
     assert d1 == d2
     for a, b in zip(s1, s2):
         assert np.array_equal(interior(a), interior(b))
 
 
 @pytest.mark.parametrize("grid", [0, 7])
-def test_staged_layout_persistent_grids(grid):
-    """The staged kernels with their default resident grid and with 7 CTAs (many
-    blocks per CTA, so every CTA refills its stage many times)."""
+def test_pair_kernels_persistent_grids(grid):
+    """The pair kernels with a CTA per block and with 7 CTAs (many blocks per CTA, each
+    assembling its tile where the one before it was)."""
     mk = lambda: cases.conical_island(128, 1)
     d1, s1 = _run(mk, 1, 0, 25)
     case = mk()
     f, _, loop = make_gpu(case)
-    f.set_kernel_layout(3)
+    f.set_kernel_layout(2)
     f.set_grid(grid)
     d3 = []
     for _ in range(25):
@@ -92,8 +97,8 @@ def test_staged_layout_persistent_grids(grid):
         assert np.array_equal(interior(a), interior(b))
 
 
-def test_staged_layout_in_a_pool():
-    """Scenarios of different sizes and step budgets in one pool with the staged
+def test_pair_kernels_in_a_pool():
+    """Scenarios of different sizes and step budgets in one pool with the pair
     kernels (finished scenarios stop swapping their state buffers while others run)
     end as each does alone with one cell per thread."""
     from bg_flood_b200.pool import ScenarioPool
@@ -105,7 +110,7 @@ def test_staged_layout_in_a_pool():
         alone.append(st)
     built = [make_gpu(mk()) for mk in mks]
     pool = ScenarioPool(mks[0]().param, sum(b[1].nblk for b in built), 4)
-    pool.set_kernel_layout(3)
+    pool.set_kernel_layout(2)
     slots = [pool.admit(f, lp, 1e30, maxsteps=n) for (f, _, lp), n in zip(built, budgets)]
     assert pool.run(64) == 0
     for slot, (f, m, _), st in zip(slots, built, alone):
@@ -143,7 +148,7 @@ SPLIT_CASES = [
 
 @pytest.mark.parametrize("name,mk,nsteps", SPLIT_CASES, ids=[c[0] for c in SPLIT_CASES])
 def test_split_layouts_bit_identical_exact(name, mk, nsteps):
-    """Split precision (FP32 deviations from per-block datums) in the two-cell kernels
+    """Split precision (FP32 deviations from per-block datums) in the pair kernels
     reproduces the one-cell split kernels bit for bit in the exact build: datum
     conversion of neighbour cells, full depths in the wet tests, the limiter and
     friction, and the datum's pressure shift."""
@@ -165,7 +170,7 @@ def test_split_layouts_close_fast(name, mk, nsteps):
 
 
 def test_split_pool_equals_alone():
-    """Two split-precision tsunami members batched in one pool (two-cell kernels,
+    """Two split-precision tsunami members batched in one pool (pair kernels,
     per-block datums in the pool's slots) end exactly as each does alone."""
     from bg_flood_b200.pool import ScenarioPool
     mks = [SPLIT_CASES[0][1], SPLIT_CASES[1][1]]
