@@ -27,7 +27,6 @@ struct M2 {
 
 __device__ __forceinline__ M2 operator&&(M2 x, M2 y) { return M2{x.a && y.a, x.b && y.b}; }
 __device__ __forceinline__ M2 operator||(M2 x, M2 y) { return M2{x.a || y.a, x.b || y.b}; }
-__device__ __forceinline__ M2 operator!(M2 x) { return M2{!x.a, !x.b}; }
 
 // ---------------------------------------------------------------- scalars
 template <class T> __device__ __forceinline__ T add(T x, T y) { return x + y; }
@@ -100,7 +99,15 @@ __device__ __forceinline__ float rcpa(float y)
 // may take the other of two products): mad always, operands of *_apart never.
 __device__ __forceinline__ float mad(float x, float y, float z) { return __fmaf_rn(x, y, z); }
 __device__ __forceinline__ double mad(double x, double y, double z) { return __fma_rn(x, y, z); }
+// (mad_sub: x y - z, sub_mad: z - x y)
+__device__ __forceinline__ float mad_sub(float x, float y, float z) { return __fmaf_rn(x, y, -z); }
+__device__ __forceinline__ double mad_sub(double x, double y, double z) { return __fma_rn(x, y, -z); }
+__device__ __forceinline__ V2<float> mad_sub(V2<float> x, V2<float> y, V2<float> z) { return mad(x, y, mul(V2<float>{-1.f, -1.f}, z)); }
+__device__ __forceinline__ float sub_mad(float z, float x, float y) { return __fmaf_rn(-x, y, z); }
+__device__ __forceinline__ double sub_mad(double z, double x, double y) { return __fma_rn(-x, y, z); }
+__device__ __forceinline__ V2<float> sub_mad(V2<float> z, V2<float> x, V2<float> y) { return mad(mul(V2<float>{-1.f, -1.f}, x), y, z); }
 __device__ __forceinline__ float sub_apart(float x, float y) { return __fsub_rn(x, y); }
+__device__ __forceinline__ double sub_apart(double x, double y) { return __dsub_rn(x, y); }
 __device__ __forceinline__ V2<float> sub_apart(V2<float> x, V2<float> y) { return sub(x, y); }
 __device__ __forceinline__ float mul_apart(float x, float y) { return __fmul_rn(x, y); }
 __device__ __forceinline__ double mul_apart(double x, double y) { return __dmul_rn(x, y); }
@@ -125,6 +132,8 @@ __device__ __forceinline__ V2<float> add(V2<float> x, V2<float> y) { return V2<f
 __device__ __forceinline__ V2<float> sub(V2<float> x, V2<float> y) { return V2<float>{__fsub_rn(x.a, y.a), __fsub_rn(x.b, y.b)}; }
 __device__ __forceinline__ V2<float> mul(V2<float> x, V2<float> y) { return V2<float>{__fmul_rn(x.a, y.a), __fmul_rn(x.b, y.b)}; }
 __device__ __forceinline__ V2<float> mad(V2<float> x, V2<float> y, V2<float> z) { return add(mul(x, y), z); }
+template <class V> __device__ __forceinline__ V mad_sub(V x, V y, V z) { return sub(mul(x, y), z); }
+template <class V> __device__ __forceinline__ V sub_mad(V z, V x, V y) { return sub(z, mul(x, y)); }
 template <class V> __device__ __forceinline__ V sub_apart(V x, V y) { return sub(x, y); }
 #endif
 
@@ -149,15 +158,6 @@ template <class T> __device__ __forceinline__ V2<T> vmax(V2<T> x, V2<T> y)
     return V2<T>{M<T>::fmax_(x.a, y.a), M<T>::fmax_(x.b, y.b)};
 }
 template <class T> __device__ __forceinline__ V2<T> vabs(V2<T> x) { return V2<T>{M<T>::fabs_(x.a), M<T>::fabs_(x.b)}; }
-template <class T> __device__ __forceinline__ T vcopysign(T x, T y)
-{
-    if constexpr (sizeof(T) == 4) return copysignf(x, y);
-    else return copysign(x, y);
-}
-template <class T> __device__ __forceinline__ V2<T> vcopysign(V2<T> x, V2<T> y)
-{
-    return V2<T>{vcopysign<T>(x.a, y.a), vcopysign<T>(x.b, y.b)};
-}
 template <class T> __device__ __forceinline__ M2 lt(V2<T> x, V2<T> y) { return M2{x.a < y.a, x.b < y.b}; }
 template <class T> __device__ __forceinline__ M2 gt(V2<T> x, V2<T> y) { return M2{x.a > y.a, x.b > y.b}; }
 template <class T> __device__ __forceinline__ M2 ge(V2<T> x, V2<T> y) { return M2{x.a >= y.a, x.b >= y.b}; }

@@ -270,9 +270,8 @@ __device__ __forceinline__ FluxQ<V> face_q(const FaceQ<V>& f, V g, V ga, V epsi,
         fu = sel(live, ful, zero);
         a = sel(live, a, zero);
         ft = mul(sel(gt(fh, zero), f.tN, f.tI), fh);
-        const V nhI = mul(mone, f.hI), nhN = mul(mone, f.hN);
-        fq = mad(nga, mad(add(f.hI, f.hsi), sub(f.zri, f.eI), mad(nhI, f.hI, mul(hp, hp))), fu);
-        s = mad(nga, mad(add(f.hN, f.hsn), sub(f.zrn, f.eN), mad(nhN, f.hN, mul(hm, hm))), fu);
+        fq = mad(nga, mad(add(f.hI, f.hsi), sub(f.zri, f.eI), sub_mad(mul(hp, hp), f.hI, f.hI)), fu);
+        s = mad(nga, mad(add(f.hN, f.hsn), sub(f.zrn, f.eN), sub_mad(mul(hm, hm), f.hN, f.hN)), fu);
     } else {
         const V zA = vmax(sub(f.eI, f.hI), sub(f.eN, f.hN));
         const V zCN = vmin(zA, vmin(f.eN, f.eI));
@@ -292,7 +291,7 @@ __device__ __forceinline__ FluxQ<V> face_q(const FaceQ<V>& f, V g, V ga, V epsi,
         const V den = sub(SR, SL);
         const V nSL = mul(mone, SL);
         const V nh = mad(SLSR, sub(hp, hm), mad(nSL, fhp, mul(SR, fhm)));
-        const V nq = mad(SLSR, mad(hp, up, mul(mone, fhm)), mad(nSL, fup, mul(SR, fum)));
+        const V nq = mad(SLSR, mad_sub(hp, up, fhm), mad(nSL, fup, mul(SR, fum)));
         V fhM, fqM;
 #if BGF_FAST
         if constexpr (sizeof(T) == 4) {
@@ -493,7 +492,7 @@ __device__ __forceinline__ void friction_v(int model, typename LaneOf<V>::T g, t
 // The two cells of ring element k (0..63) of a block's tile, as cells k and k + 64: for
 // k < 32 the ring columns -1, -2, 16, 17 at rows (k & 7) and (k & 7) + 8, beyond them the
 // ring rows (-1, 16) and (-2, 17) at column k & 15.  Gives the cell's tile position and its
-// source (ring_src2).
+// source.
 template <class T>
 __device__ __forceinline__ void ring_cell(const DevModel<T>& m, int ib, int k, int& x, int& y, int& sb, int& sx, int& sy)
 {
@@ -612,16 +611,25 @@ __device__ __forceinline__ void store_ring(SmemQ<T, LANES>& s, int x, int y, T h
     if (x >= -1 && x <= BW && y >= -1 && y <= BW) BGF_ROW(s.zb, pz, x, y) = z;
 }
 
-// 1 + x / y.  Fast FP32 build: the product with the reciprocal fused into the sum.
-template <class V> __device__ __forceinline__ V one_plus_quot(V x, V y)
+// 1 + x / y and 1 - x / y.  Fast FP32 build: the product with the reciprocal fused into the sum.
+template <class V> __device__ __forceinline__ void one_pm_quot(V x, V y, V& plus, V& minus)
 {
     using T = typename LaneOf<V>::T;
     const V one = cst<V>((T)1.0);
 #if BGF_FAST
-    if constexpr (sizeof(T) == 4) return mad(x, rcp_v(y), one);
-    else return add_apart(one, dv(x, y));
+    if constexpr (sizeof(T) == 4) {
+        const V r = rcp_v(y);
+        plus = mad(x, r, one);
+        minus = mad(mul(cst<V>((T)-1.0), x), r, one);
+    } else {
+        const V q = dv(x, y);
+        plus = add_apart(one, q);
+        minus = sub_apart(one, q);
+    }
 #else
-    return add(one, dv(x, y));
+    const V q = dv(x, y);
+    plus = add(one, q);
+    minus = sub(one, q);
 #endif
 }
 
@@ -643,9 +651,10 @@ __device__ __forceinline__ void both_sides(V dx, V h, V zs, V un, V ut, V gh, V 
         lo.e = mad(ndx, gz, zs);
         hi.e = mad(dx, gz, zs);
         const auto wet = gt(Hfull, epsv);
-        const V dh = mul(dx, gh);
-        const V cl = sel(wet, mul(one_plus_quot(dh, Hfull), ndx), ndx);
-        const V ch = sel(wet, mul(one_plus_quot(mul(cst<V>((T)-1.0), dh), Hfull), dx), dx);
+        V lowq, highq;
+        one_pm_quot<V>(mul(dx, gh), Hfull, lowq, highq);
+        const V cl = sel(wet, mul(lowq, ndx), ndx);
+        const V ch = sel(wet, mul(highq, dx), dx);
         lo.n = mad(cl, gn, un);
         lo.t = mad(cl, gt_, ut);
         hi.n = mad(ch, gn, un);
@@ -747,7 +756,9 @@ __device__ __forceinline__ T tile_faces(SmemQ<T, LANES>& s, const StepParams<T>&
             if (part == 0) {
                 g1 = wetslope_v<T>(hd_s, n1, Hr, f1, i1, g1, g0, bg.ring);
                 // the velocities' factor (both_sides)
-                c1 = sel(gt(Hr, p.epsface), mul(one_plus_quot(-mul(hd_s, g0), Hr), hd_s), hd_s);
+                T lowq, highq;
+                one_pm_quot<T>(mul(hd_s, g0), Hr, lowq, highq);
+                c1 = sel(gt(Hr, p.epsface), mul(highq, hd_s), hd_s);
             }
             c1 = __shfl_sync(0xffffffffu, c1, lane & ~1);
             if (part == 0) c1 = hd_s;
