@@ -43,13 +43,6 @@ namespace BGF_VARIANT {
 #include "bgf_pair.cuh"
 #include "bgf_quad.cuh"
 
-__device__ __forceinline__ bool has_coarser_side(const int* nbr, int nbm, const int* lv, int ib)
-{
-    const int l = lv[ib];
-    return lv[nbr[0 * nbm + ib]] < l || lv[nbr[2 * nbm + ib]] < l || lv[nbr[4 * nbm + ib]] < l ||
-           lv[nbr[6 * nbm + ib]] < l;
-}
-
 __device__ __forceinline__ bool has_finer_neighbour(const int* nbr, int nbm, const int* lv, int ib)
 {
     const int l = lv[ib];
@@ -396,7 +389,8 @@ template <class T> struct AmrOcc {
     static constexpr int step = sizeof(T) == 4 ? 6 : 3;
 };
 
-// Cells of a pair that a thread of the flux kernel owns (as quad_lanes in bgf_flow.cu).
+// Cells of a pair that a thread of the step kernel owns: one in FP64, a pair in FP32 on every
+// mesh (quad_lanes in bgf_flow.cu also takes one cell on small meshes of the exact build).
 template <class T> __host__ __device__ constexpr int amr_lanes() { return sizeof(T) == 8 ? 1 : 2; }
 
 // Fluxes and update of a chain's blocks, in the layout of the single-level kernels

@@ -237,7 +237,7 @@ int bgf_flow_step_noalloc(const bgf_param* p, const bgf_noalloc_args* a, bgf_loo
         !a->h_out || !a->u_out || !a->v_out)
         return BGF_EINVAL;
     if (p->engine == 1 && (!a->dzbdx || !a->dzbdy)) return BGF_EINVAL;
-    // (the interface asks for 16 bytes, which wider bed loads may rely on)
+    // (a rule of the interface; the present kernels load the bed value by value)
     if (((uintptr_t)a->zb & 15) != 0) {
         bgf::set_last_error("zb must be 16-byte aligned (as cudaMalloc returns it)");
         return BGF_EINVAL;
