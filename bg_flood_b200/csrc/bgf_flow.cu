@@ -360,6 +360,10 @@ template <class T> __global__ void volume_kernel(DevModel<T> m, T delta0, int cu
 
 // ---------------------------------------------------------------- launchers
 
+// Five blocks of the exact build fit an SM with one cell per thread: up to 740 blocks they are
+// one wave on 148 SMs, beyond it a second begins.  us per step (lake, B200), one cell a thread
+// against pairs: 64 blocks 18.0 / 20.6, 425 26.3 / 28.9, 576 30.7 / 31.0, 676 33.7 / 33.8,
+// 784 42.0 / 36.1, 1,024 48.7 / 39.4, 1,280 56.9 / 56.0, 1,600 68.5 / 64.2.
 constexpr int kOneCellBlocks = 700;
 
 template <class T> size_t smem_bytes() { return sizeof(Smem<T>); }
@@ -367,7 +371,7 @@ template <class T> size_t smem_bytes() { return sizeof(Smem<T>); }
 // Cells of a pair that a thread of the step kernels owns on a mesh of n blocks.  FP64: one
 // (20 % faster at every size, 100 to 3000 blocks, than one pair: 24 instead of 12 warps per
 // SM).  FP32, fast build: a pair (one cell is 20 to 100 % slower).  FP32, exact build: one
-// cell where the blocks leave the SMs short of warps.
+// cell where the blocks are one wave (kOneCellBlocks).
 template <class T> constexpr int quad_lanes(int n)
 {
 #if BGF_FAST

@@ -36,9 +36,9 @@
 // their order and is bit-identical to them.
 //
 // Measured against the kernels this replaced (pairs of adjacent rows, faces from gradients)
-// on B200: 545 -> 477 thread-instructions per cell in the predictor and 633 -> 579 in the
-// corrector (fast FP32); with the chained launches (pdl_trigger) the step of the 1024x1024
-// run-up takes 51.9 instead of 56.6 us, of a 4096x4096 one 729 instead of 769 us.  Two
+// on B200: 545 -> 525 warp-instructions x 32 per cell in the predictor and 633 -> 635 in the
+// corrector (fast FP32); with even shares of the work and the chained launches (pdl_trigger) the step of the 1024x1024
+// run-up takes 51.8 instead of 56.6 us, of a 4096x4096 one 729 instead of 769 us.  Two
 // pairs per thread (398 and 503 instructions per cell, 128 registers) ran as fast on large
 // grids and slower on all others; one warp marching over a block's rows (no barriers) was
 // half as fast, its warps out of step in the instruction cache.
@@ -527,8 +527,8 @@ __device__ __forceinline__ void ring_cell(const DevModel<T>& m, int ib, int k, i
 
 // Whether the slopes of the ring are spread over threads 0..127 (two a ring cell) instead of
 // made by two warps: the exact build's are long enough to
-// keep the other warps waiting (12,288 blocks: 426 instead of 453 us per step), the fast
-// build's are not (146 instead of 142 us).
+// keep the other warps waiting (12,288 blocks: 426 instead of 453 us per step when this was
+// chosen), the fast build's are not (151 instead of 148 us).
 template <class T, int LANES> struct RingPass {
 #if BGF_FAST
     static constexpr bool spread = false;
@@ -888,8 +888,9 @@ __device__ __forceinline__ T tile_faces(SmemQ<T, LANES>& s, const StepParams<T>&
     }
     // the faces on the right column (pairs of rows) and the top row (pairs of columns)
     // (one face a lane: with a pair in each of half the lanes the other warps wait longer,
-    // 428 instead of 408 us per step for 12,288 blocks of the exact build, 152 instead of
-    // 147 us in split precision)
+    // 428 instead of 408 us per step for 12,288 blocks of the exact build, fast build
+    // 740 instead of 729 us for 65,536 blocks, 25.0 instead of 23.9 us in split precision
+    // for 1,536; face_q has the same roundings in both forms)
     if (at.extra) {
         const bool isx = (lane & 15) < 8;
         const int q = lane & 7, el = lane >> 4;  // (which of the two cells)

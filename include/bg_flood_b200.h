@@ -187,7 +187,8 @@ int bgf_flow_step(bgf_handle* h, bgf_loop* loop);
  * (if > 0) each time it is reached.  On return loop holds the final state
  * of the time loop and *nsteps the number of steps taken.
  * Returns BGF_EDT_UNDERFLOW if dt < dtmin before endtime (CrashDetection,
- * src/Mainloop.cu:648-719). */
+ * src/Mainloop.cu:648-719).  If a CUDA call fails after some steps ran, loop and
+ * *nsteps say how far the device got. */
 int bgf_run(bgf_handle* h, bgf_loop* loop, double endtime, double outputtimestep, int maxsteps,
             int* nsteps);
 
